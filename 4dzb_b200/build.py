@@ -19,7 +19,8 @@ LIB = os.path.join(HERE, "libfdzb.so")
 
 SOURCES = ["fdzb_pipeline.cu", "fdzb_shade.cu", "fdzb_raster.cu", "fdzb_api.cpp", "fdzb_serve.cpp",
            "fdzb_light.cpp"]
-HEADERS = ["fdzb_internal.h", "fdzb_engine.h", "fdzb_device.cuh", "fdzb_sort.cuh", "fdzb_occlusion.cuh"]
+HEADERS = ["fdzb_internal.h", "fdzb_engine.h", "fdzb_device.cuh", "fdzb_sort.cuh", "fdzb_occlusion.cuh",
+           "fdzb_edge_masks.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

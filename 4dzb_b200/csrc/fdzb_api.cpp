@@ -113,7 +113,7 @@ size_t layout(fdzb::DeviceBuffers &b, char *base, int nf, long long S, long long
     b.binSampleEnd = (int32_t *)take(4 * ((size_t)NB + 1));
     b.binStat = (uint32_t *)take(32 * (size_t)NB);
     b.triRec = (float4 *)take(64 * Ts);
-    b.triPrj = (float4 *)take(32 * Ts);
+    b.triFast = (float4 *)take(64 * Ts);
     b.triCount = (int32_t *)take(4 * Ts);
     b.triScanStatus = (unsigned long long *)take(8 * ((Ts + fdzb::kTriTileHost - 1) / fdzb::kTriTileHost));
     b.tkeysA = (uint32_t *)take(4 * Ts);
@@ -346,22 +346,17 @@ int engine_enqueue(Engine &e)
     for (const FrameSpec &f : e.frames) {
         wide = wide || f.light.N > fdzb::kMaxLightN32 || f.light.NC > fdzb::kMaxLightN32;
         square = square && f.light.N == f.light.NC;
-        rows16 = rows16 && f.light.N <= 16;
+        rows16 = rows16 && f.light.N <= 16 && f.light.NC <= 31;
     }
     b.wide = wide ? 1 : 0;
     b.rows16 = rows16 ? 1 : 0;
     b.depthPlane = e.depthPlane;
     b.rayCast = e.rayCast;
     b.occVariant = (e.occVariant == 1 && !wide && square && !e.depthPlane) ? 1 : 0;
-    {
-        e.lastShape = std::make_tuple(nf, S, T, NB);
-        const auto known = e.openBoxKeep.find(e.lastShape);   // a shape not seen yet: probe the cull
-        const bool want = e.openBoxMode == FDZB_OPEN_BOX_ON ||
-                          (e.openBoxMode == FDZB_OPEN_BOX_AUTO && (known == e.openBoxKeep.end() || known->second));
-        b.openBox = (want && !e.rayCast && b.occVariant == 0) ? 1 : 0;
-        b.countWork = (e.profile && e.countWork) ? 1 : 0;
-        e.lastOpenBox = b.openBox != 0;
-    }
+    // the open-box cull pays or costs nothing on every frame measured
+    // (fdzb_edge_masks.cuh), so auto means on
+    b.openBox = (e.openBoxMode != FDZB_OPEN_BOX_OFF && !e.rayCast && b.occVariant == 0) ? 1 : 0;
+    b.countWork = (e.profile && e.countWork) ? 1 : 0;
     // Triangle lists: the pairs are sorted by bin only (stable, so a bin lists
     // its triangles in the order the pairs were emitted,
     // K/Step4_RasterizeTriangleToBin.inl:220-223).  Reference order emits them by
@@ -644,11 +639,6 @@ int engine_sync(Engine &e)
     FDZB_CUDA(cudaEventElapsedTime(&ms, e.ev0, e.ev1));
     e.lastMs = ms;
     e.passes = 1;
-    if (e.lastOpenBox && e.openBoxMode == FDZB_OPEN_BOX_AUTO && !e.openBoxKeep.count(e.lastShape)) {
-        const fdzb::Counters &k = *e.hCounters;
-        const double rate = k.pairsExamined ? (double)k.boxSkips / (double)k.pairsExamined : 0.0;
-        e.openBoxKeep[e.lastShape] = rate >= kOpenBoxKeep;
-    }
     return FDZB_OK;
 }
 
@@ -1139,7 +1129,6 @@ int fdzb_ctx_set_open_box(fdzb_ctx *c, int mode)
         return fail(FDZB_ERR_INVALID_ARG, "open-box mode: FDZB_OPEN_BOX_OFF, _ON or _AUTO");
     if (int rc = ctx_sync(c)) return rc;
     c->eng.openBoxMode = mode;
-    c->eng.openBoxKeep.clear();
     return FDZB_OK;
 }
 
@@ -1150,7 +1139,6 @@ int fdzb_batch_set_open_box(fdzb_batch *b, int mode)
         return fail(FDZB_ERR_INVALID_ARG, "open-box mode: FDZB_OPEN_BOX_OFF, _ON or _AUTO");
     if (int rc = engine_sync(b->eng)) return rc;
     b->eng.openBoxMode = mode;
-    b->eng.openBoxKeep.clear();
     return FDZB_OK;
 }
 

@@ -30,6 +30,11 @@ struct LightParams {
     int NC;                 // columns (lightResHeight)
     uint32_t full;          // NC low bits set, when NC <= 32
     unsigned long long fullRows, fullCols;  // N and NC low bits set
+    // Light-grid coordinates of a point V (fdzb_edge_masks.cuh): G (V - ur), G
+    // the inverse of the columns (xd, yd, unit normal towards the scene), and
+    // the constants of the fast pair test's error bound (FastConst).
+    double G[9];
+    float fc[8];
 };
 
 // Per-frame inputs, outputs and batch offsets (host-filled).
@@ -124,7 +129,7 @@ struct DeviceBuffers {
     uint32_t *binStat;                          // [8 * totalBins] ordered encodings: maxz, Rx, Ry, Rz, Rw, 3 pad
     // triangles
     float4 *triRec;                             // [4 * totalTris]
-    float4 *triPrj;                             // [2 * totalTris] vertex projections (open-box test)
+    float4 *triFast;                            // [4 * totalTris] the edge-mask kernel's records (FastTri)
     int32_t *triCount;                          // [totalTris]
     unsigned long long *triScanStatus;          // [triTiles] epoch-tagged look-back words
     // pairs
@@ -153,7 +158,7 @@ struct DeviceBuffers {
     int depthPlane;                             // 1: the frames test each triangle's own plane
     int openBox;                                // 1: the occlusion kernel with the open-box cull
     int countWork;                              // 1: the occlusion kernel that accumulates the work counters
-    int rows16;                                 // 1: every grid of the launch has at most 16 rows
+    int rows16;                                 // 1: every grid of the launch has at most 16 rows of at most 31 columns
     uint32_t *epochWord;                        // launch sequence number (look-back tags), advanced
                                                 // on the device by k_init so graph replays stay fresh
     // debug capture (nullptr unless enabled): pre-sort copies of the key/value arrays

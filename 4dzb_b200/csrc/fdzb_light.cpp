@@ -37,6 +37,41 @@ inline void put(float *d, V3 a)
     d[2] = a.z;
 }
 
+// Light-grid coordinates and the fast pair test's constants (fdzb_edge_masks.cuh
+// has the bound they come from; u = 2^-24).  A light whose grid spans no plane,
+// or whose steps are so small or large that the bound would have to count
+// underflow or overflow, keeps the zero matrix: no sample then lies in front of
+// the light, which sends every pair to the reference's test.
+void grid_frame(LightParams *L, V3 view)
+{
+    const double x[3] = {L->xd[0], L->xd[1], L->xd[2]}, y[3] = {L->yd[0], L->yd[1], L->yd[2]};
+    const double c[3] = {x[1] * y[2] - x[2] * y[1], x[2] * y[0] - x[0] * y[2], x[0] * y[1] - x[1] * y[0]};
+    const double len = std::sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
+    const double facing = c[0] * view.x + c[1] * view.y + c[2] * view.z;
+    const double sx = std::sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+    const double sy = std::sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
+    const double u = 1.0 / 16777216.0;
+    if (!(len > 1e-3 * sx * sy) || !std::isfinite(len) || facing == 0.0 || !std::isfinite(facing)) return;
+    if (!(std::fmin(sx, sy) >= 1e-8 && std::fmax(sx, sy) <= 1e5)) return;
+    const double z[3] = {c[0] / (facing > 0 ? len : -len), c[1] / (facing > 0 ? len : -len),
+                         c[2] / (facing > 0 ? len : -len)};
+    // rows of the inverse of (x y z): cross products over the determinant
+    const double vol = c[0] * z[0] + c[1] * z[1] + c[2] * z[2];
+    const double *col[3] = {x, y, z};
+    for (int i = 0; i < 3; ++i) {
+        const double *p = col[(i + 1) % 3], *q = col[(i + 2) % 3];
+        L->G[3 * i] = (p[1] * q[2] - p[2] * q[1]) / vol;
+        L->G[3 * i + 1] = (p[2] * q[0] - p[0] * q[2]) / vol;
+        L->G[3 * i + 2] = (p[0] * q[1] - p[1] * q[0]) / vol;
+    }
+    const double av = std::fabs(vol);
+    L->fc[0] = (float)(sx * 1.0001);
+    L->fc[1] = (float)(sy * 1.0001);
+    L->fc[2] = (float)((L->N * sx + L->NC * sy) * 1.0001);
+    L->fc[3] = (float)(11.0 * u / av);
+    L->fc[4] = (float)(1.002 / av);
+}
+
 }  // namespace
 
 void light_setup(const float rightRadius, const float topRadius, const float position[3],
@@ -104,6 +139,7 @@ void light_setup(const float rightRadius, const float topRadius, const float pos
         }
     L->RF[0] = rightRadius * 2.0f * xf * P[0][0] * 0.5f;
     L->RF[1] = topRadius * 2.0f * yf * P[1][1] * 0.5f;
+    grid_frame(L, view);
 }
 
 }  // namespace fdzb

@@ -23,7 +23,7 @@
 //                 sample, OR-accumulating N-bit row masks.
 #include "fdzb_device.cuh"
 #include "fdzb_sort.cuh"
-#include "fdzb_occlusion.cuh"
+#include "fdzb_edge_masks.cuh"
 
 #include <mutex>
 #include <string>
@@ -240,15 +240,38 @@ __global__ void k_plan(const FrameDesc *__restrict__ frames, FrameState *states,
 
 // ---------------------------------------------------------------------------
 // k_tri_setup: grid (x, frame).  Record layout (4 x float4 = 64 B):
-//   q0 = (v0, minz) q1 = (v1, maxz) q2 = (v2, 1/w2) q3 = (aabb min x,y, aabb max x,y)
-// and the vertices' projections for the occlusion stage's open-box test
-// (2 x float4): (u0, v0, 1/w0, u1), (v1, 1/w1, u2, v2).
+//   q0 = (v0, minz) q1 = (v1, maxz) q2 = (v2, 0) q3 = (aabb min x,y, aabb max x,y)
+// and the edge-mask kernel's record (FastTri, 4 x float4).
 // Culled triangles keep the inverted AABB of the reference's triAABB buffer, so
 // the pair counter's skip test rejects them exactly as K/Step4_*.inl:41 does.
 // ---------------------------------------------------------------------------
+// The fast record of a triangle that was not culled (FastTri).
+__device__ __forceinline__ void store_fast_tri(float4 *__restrict__ o, const LightParams &L, f3 v0, f3 v1, f3 v2,
+                                               float4 aabb, float minz, float maxz)
+{
+    const f3 e0 = sub3(v0, v1), e1 = sub3(v1, v2), e2 = sub3(v2, v0);
+    const float E = sqrtf(fmaxf(fmaxf(dot3(e0, e0), dot3(e1, e1)), dot3(e2, e2))) * 1.0001f;
+    const f3 a = light_grid_coords(L, v0), b = light_grid_coords(L, v1), c = light_grid_coords(L, v2);
+    if (!(in_range(a) && in_range(b) && in_range(c))) {
+        // no vertex of it counts as above a sample: every pair goes to pair_test
+        const float inf = __int_as_float(0x7f800000);
+        o[0] = aabb;
+        o[1] = make_float4(minz, inf, 0.0f, 0.0f);
+        o[2] = make_float4(inf, 0.0f, 0.0f, inf);
+        o[3] = make_float4(0.0f, 0.0f, inf, inf);
+        return;
+    }
+    const bool front = minz > 0.0f && a.z > 0.0f && b.z > 0.0f && c.z > 0.0f;
+    const float S = max3(max3(fabsf(a.x), fabsf(b.x), fabsf(c.x)), max3(fabsf(a.y), fabsf(b.y), fabsf(c.y)), 1.0f);
+    o[0] = aabb;
+    o[1] = make_float4(minz, E, a.x, a.y);
+    o[2] = make_float4(a.z, b.x, b.y, b.z);
+    o[3] = make_float4(c.x, c.y, c.z, front ? maxz : -S);
+}
+
 __global__ void __launch_bounds__(256)
     k_tri_setup(const FrameDesc *__restrict__ frames, FrameState *states, float4 *__restrict__ rec,
-                float4 *__restrict__ prj, int *err)
+                float4 *__restrict__ fast, int *err)
 {
     const FrameDesc &fr = frames[blockIdx.y];
     FrameState &st = states[blockIdx.y];
@@ -269,7 +292,6 @@ __global__ void __launch_bounds__(256)
                       i2 = fr.idx[3 * (size_t)t + 2];
             float mnx = kF32Max, mny = kF32Max, mnz = kF32Max;
             float mxx = -kF32Max, mxy = -kF32Max, mxz = -kF32Max;
-            float pu[3] = {0.f, 0.f, 0.f}, pv[3] = {0.f, 0.f, 0.f}, pw[3] = {0.f, 0.f, 0.f};
             f3 v0 = mk3(0.f, 0.f, 0.f), v1 = v0, v2 = v0;
             const bool okIdx = i0 >= 0 && i0 < fr.V && i1 >= 0 && i1 < fr.V && i2 >= 0 && i2 < fr.V;
             if (!okIdx) {
@@ -291,9 +313,6 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const f3 r = light_project(M, vv[k]);
-                        pu[k] = r.x;
-                        pv[k] = r.y;
-                        pw[k] = __frcp_rn(r.z);
                         mnx = fminf(mnx, r.x);
                         mny = fminf(mny, r.y);
                         mnz = fminf(mnz, r.z);
@@ -307,11 +326,9 @@ __global__ void __launch_bounds__(256)
             float4 *o = rec + 4 * (size_t)(fr.triBase + t);
             o[0] = make_float4(v0.x, v0.y, v0.z, mnz);
             o[1] = make_float4(v1.x, v1.y, v1.z, mxz);
-            o[2] = make_float4(v2.x, v2.y, v2.z, pw[2]);
+            o[2] = make_float4(v2.x, v2.y, v2.z, 0.0f);
             o[3] = make_float4(mnx, mny, mxx, mxy);
-            float4 *pp = prj + 2 * (size_t)(fr.triBase + t);
-            pp[0] = make_float4(pu[0], pv[0], pw[0], pu[1]);
-            pp[1] = make_float4(pv[1], pw[1], pu[2], pv[2]);
+            if (mnx <= mxx) store_fast_tri(fast + 4 * (size_t)(fr.triBase + t), fr.light, v0, v1, v2, o[3], mnz, mxz);
         }
         const unsigned b = __ballot_sync(kFullWarp, inLP);
         if (lane == 0 && b) atomicAdd(&st.nValidTris, __popc(b));
@@ -896,7 +913,7 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     }
     k_plan<<<(nf + 63) / 64, 64, 0, s>>>(b.frames, b.states, nf);
     k_tri_setup<<<dim3(grid_for(maxT, 256, sm * 8), nf), 256, 0, s>>>(b.frames, b.states, b.triRec,
-                                                                      b.triPrj, &b.counters->errorFlags);
+                                                                      b.triFast, &b.counters->errorFlags);
     k_sample_keys<<<dim3(grid_for(maxS, 256, sm * 8), nf), 256, 0, s>>>(
         b.frames, b.states, b.keysA, b.valsA, b.binStat, b.totalBins);
     nl += 5;
@@ -971,47 +988,47 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     // plane (the host falls back to lane per sample otherwise)
     typedef RowWord<u64> W64;
     const int g32 = sm * FDZB_OCC_MINBLOCKS, g64 = sm * W64::kMinBlocks, t64 = W64::kWarps * 32;
-#define FDZB_OCC_ARGS                                                                                        \
+#define FDZB_OCC_LISTS                                                                                       \
     b.frames, b.states, b.items, b.itemCapacity, b.counters, sv, b.binSampleStart, b.binSampleEnd, b.binTriStart, \
-        b.binTriEnd, pv, triMask, b.triRec, b.triPrj, b.totalTris, b.totalBins, nf
-    // b.openBox: the open-box cull's instantiation (edge-function masks only);
-    // b.countWork: the instantiation that accumulates the work counters
-#define FDZB_OCC(RC, RT, DP, BX, G, T)                                                                        \
-    do {                                                                                                   \
-        if (b.countWork) k_occlusion<RC, RT, DP, BX, 1><<<G, T, 0, s>>>(FDZB_OCC_ARGS);                     \
-        else k_occlusion<RC, RT, DP, BX, 0><<<G, T, 0, s>>>(FDZB_OCC_ARGS);                                 \
+        b.binTriEnd, pv, triMask, b.triRec
+    // b.openBox: the open-box cull's instantiation; b.countWork: the one that
+    // accumulates the work counters; b.rows16: grids of at most 16 rows, the
+    // lanes' masks in 16-row shared arrays
+#define FDZB_OCC(RT, DP, BX, ROWS, G, T)                                                                      \
+    do {                                                                                                     \
+        if (b.countWork)                                                                                     \
+            k_occlusion<RT, DP, BX, 1, ROWS><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
+        else                                                                                                 \
+            k_occlusion<RT, DP, BX, 0, ROWS><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
     } while (0)
-    // grids of at most 16 rows: the lanes' masks in 16-row shared arrays
-#define FDZB_OCC16(DP, BX)                                                                                    \
-    do {                                                                                                   \
-        if (b.countWork) k_occlusion<0, uint32_t, DP, BX, 1, 16><<<g32, kOccThreads, 0, s>>>(FDZB_OCC_ARGS); \
-        else k_occlusion<0, uint32_t, DP, BX, 0, 16><<<g32, kOccThreads, 0, s>>>(FDZB_OCC_ARGS);             \
+#define FDZB_OCC_FORMS(RT, ROWS, G, T)                                                                        \
+    do {                                                                                                     \
+        if (b.depthPlane && b.openBox) FDZB_OCC(RT, 1, 1, ROWS, G, T);                                        \
+        else if (b.depthPlane) FDZB_OCC(RT, 1, 0, ROWS, G, T);                                                \
+        else if (b.openBox) FDZB_OCC(RT, 0, 1, ROWS, G, T);                                                   \
+        else FDZB_OCC(RT, 0, 0, ROWS, G, T);                                                                  \
     } while (0)
-    if (b.wide) {
-        if (b.rayCast) FDZB_OCC(1, u64, 0, 0, g64, t64);
-        else if (b.depthPlane && b.openBox) FDZB_OCC(0, u64, 1, 1, g64, t64);
-        else if (b.depthPlane) FDZB_OCC(0, u64, 1, 0, g64, t64);
-        else if (b.openBox) FDZB_OCC(0, u64, 0, 1, g64, t64);
-        else FDZB_OCC(0, u64, 0, 0, g64, t64);
-    } else if (b.rayCast) {
-        FDZB_OCC(1, uint32_t, 0, 0, g32, kOccThreads);
+#define FDZB_RAYCAST(RT, G, T)                                                                                \
+    do {                                                                                                     \
+        if (b.countWork) k_raycast<RT, 1><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.totalTris, b.totalBins, nf);      \
+        else k_raycast<RT, 0><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.totalTris, b.totalBins, nf);                  \
+    } while (0)
+    if (b.rayCast) {
+        if (b.wide) FDZB_RAYCAST(u64, g64, t64);
+        else FDZB_RAYCAST(uint32_t, g32, kOccThreads);
+    } else if (b.wide) {
+        FDZB_OCC_FORMS(u64, 64, g64, t64);
     } else if (b.occVariant == 1) {
-        k_occlusion_pairs<<<sm * FDZB_OCC2_MINBLOCKS, kOccThreads, 0, s>>>(FDZB_OCC_ARGS);
-    } else if (b.depthPlane) {
-        if (b.openBox && b.rows16) FDZB_OCC16(1, 1);
-        else if (b.openBox) FDZB_OCC(0, uint32_t, 1, 1, g32, kOccThreads);
-        else if (b.rows16) FDZB_OCC16(1, 0);
-        else FDZB_OCC(0, uint32_t, 1, 0, g32, kOccThreads);
-    } else if (b.openBox) {
-        if (b.rows16) FDZB_OCC16(0, 1);
-        else FDZB_OCC(0, uint32_t, 0, 1, g32, kOccThreads);
+        k_occlusion_pairs<<<sm * FDZB_OCC2_MINBLOCKS, kOccThreads, 0, s>>>(FDZB_OCC_LISTS, b.totalTris, b.totalBins, nf);
+    } else if (b.rows16) {
+        FDZB_OCC_FORMS(uint32_t, 16, g32, kOccThreads);
     } else {
-        if (b.rows16) FDZB_OCC16(0, 0);
-        else FDZB_OCC(0, uint32_t, 0, 0, g32, kOccThreads);
+        FDZB_OCC_FORMS(uint32_t, 32, g32, kOccThreads);
     }
+#undef FDZB_RAYCAST
+#undef FDZB_OCC_FORMS
 #undef FDZB_OCC
-#undef FDZB_OCC16
-#undef FDZB_OCC_ARGS
+#undef FDZB_OCC_LISTS
     nl += 2;
     if (ev) cudaEventRecord(ev[STAGE_COUNT], s);
     if (launches) *launches = nl;
@@ -1062,12 +1079,46 @@ cudaError_t measure_alu_rate(double *rate)
     return e;
 }
 
+// a / b rounded to nearest, from y = RN(1/b): two correction steps of
+// Markstein's method (P. Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990, with the
+// theorem as restated in Muller et al., Handbook of Floating-Point
+// Arithmetic, sec. 4.7).  With a, b, y free of underflow and overflow:
+// q0 = RN(a y) lies within two ulps of a/b, so each residual a - b q is exact
+// (an FMA); the first step brings q within one ulp (in fact within half an
+// ulp plus a term of order 2^-46), and the second, by Markstein's theorem (y
+// within half an ulp of 1/b, q within one ulp of a/b), returns RN(a/b).  A
+// quotient then costs five FP32 operations instead of a division; the device
+// self-check (fdzb_check_division) compares it with the IEEE division.
+__device__ __forceinline__ float div_by_rcp(float a, float b, float y)
+{
+    const float q0 = __fmul_rn(a, y);
+    const float r0 = __fmaf_rn(-b, q0, a);
+    const float q1 = __fmaf_rn(r0, y, q0);
+    const float r1 = __fmaf_rn(-b, q1, a);
+    return __fmaf_rn(r1, y, q1);
+}
+
+// RN(1/b) for normal b with |b| in [2^-100, 2^40): the hardware's approximate
+// reciprocal (rcp.approx) and one Newton-Raphson step in FMA form,
+// y1 = y0 + y0 (1 - b y0) (the iteration of Markstein's paper above and of
+// Muller et al., sec. 4.7).  On that range the result equals the correctly
+// rounded reciprocal (__frcp_rn) for every one of its 2^23 x 140 x 2 values,
+// which the device self-check (fdzb_check_division) enumerates.
+__device__ __forceinline__ float rcp_nearest(float b)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(y, __fmaf_rn(-b, y, 1.0f), y);
+}
+
 // ---------------------------------------------------------------------------
-// Self-check of the occlusion rows' quotient.  k_check_reciprocal enumerates
+// Self-check of a row quotient from a hoisted reciprocal against the division
+// that the reference's rows (and pair_test) take.  k_check_reciprocal enumerates
 // every float b with |b| in [2^-100, 2^40) (both signs) and compares
 // rcp_nearest(b) with __frcp_rn(b).  k_check_division compares
 // div_by_rcp(a, b, rcp_nearest(b)) with the IEEE division __fdiv_rn, over
-// the operand ranges the pair test admits to it.
+// the operand ranges in which nothing underflows or overflows.
 // Trial t draws (from a counter hash of seed and t) three cases: a and b with
 // random significands and signs, |a| in [2^-61, 2^47] and |b| in
 // [2^-100, 2^39] (quotients outside [2^-100, 2^100] are skipped); a quotient

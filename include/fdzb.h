@@ -284,10 +284,9 @@ int fdzb_ctx_set_profiling(fdzb_ctx *ctx, int enable);
  * occlusion kernel's operation rate is reported.  No counterpart in the reference. */
 int fdzb_measure_alu_rate(double *lane_ops_per_second);
 
-/* Device self-check of the occlusion kernel's row quotient: -D / B from a
- * hoisted reciprocal RN(1/B) by two Markstein correction steps, which the pair
- * test uses in place of the IEEE division where its operands are in range,
- * the reciprocal itself from the hardware approximation and one
+/* Device self-check of a row quotient -D / B from a hoisted reciprocal RN(1/B)
+ * by two Markstein correction steps, the reciprocal itself from the hardware
+ * approximation and one
  * Newton-Raphson step.  Compares that reciprocal with __frcp_rn for every
  * float of the admitted range (|B| in [2^-100, 2^40), 2.35e9 values), then
  * runs `trials` trials of three cases each (random operands over the admitted
@@ -415,13 +414,9 @@ int fdzb_ctx_set_occlusion_shape(fdzb_ctx *ctx, int chunk, int item);
 /* Open-box cull, no counterpart in the reference: once some of a sample's
  * light rows or columns are full, a pair whose triangle cannot reach the box
  * of its still-unset light samples (a test on the triangle's projected
- * vertices, with a margin far above FP32 rounding) is skipped; masks and
- * shadows are identical (the mask is the OR over the bin's triangles).  It
- * runs in its own instantiation of the occlusion kernel, which is faster where
- * samples end in umbra and slower where they stay in penumbra.  AUTO (the
- * default): the first launch of each launch shape (frames, samples, triangles,
- * bins) runs it and counts the staged pairs it skips; the shape keeps it only
- * if that is at least a quarter of them.  Edge-function masks only. */
+ * vertices, with a margin above the FP32 rounding of its edges) is skipped;
+ * masks and shadows are identical (the mask is the OR over the bin's
+ * triangles).  AUTO (the default) is ON.  Edge-function masks only. */
 #define FDZB_OPEN_BOX_OFF 0
 #define FDZB_OPEN_BOX_ON 1
 #define FDZB_OPEN_BOX_AUTO 2
