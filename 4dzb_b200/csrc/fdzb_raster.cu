@@ -16,12 +16,12 @@
 //
 // B200 layout: one thread per triangle sets up at most two sub-triangles (the
 // near-plane clip of a triangle is a triangle or a quad) into 144-byte records
-// at slots 2t and 2t+1, and counts the 16 x 16 pixel tiles their pixel boxes
-// touch; an exclusive scan over tiles sizes the tile lists; a scatter fills
-// them; one 256-thread block per non-empty tile stages its list 32 records at
-// a time in shared memory and keeps, per pixel (one thread each), the least
-// (depth, slot) -- the GL_LESS winner whatever the order of evaluation -- and
-// finally resolves the winner's attributes.
+// at slots 2t and 2t+1, with the 16 x 16 pixel tiles their pixel boxes touch (8
+// bytes a slot), and counts the tiles' lists; the lists are laid out (k_rs_lists)
+// and filled (k_rs_scatter); one 256-thread block per tile resolves its pixels
+// and writes each once, cleared or drawn.  Nothing waits on the host: a draw
+// whose lists outgrow their buffer reads the slots' tile boxes instead of the
+// lists (k_rs_tiles), and the next draw finds a larger buffer.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,11 +37,16 @@ namespace {
 
 constexpr int kTile = 16;              // pixels per tile side
 constexpr int kRecF4 = 9;              // float4s per sub-triangle record
-constexpr int kChunk = 32;             // records staged per round
+constexpr int kChunk = kTile * kTile;  // records staged per round, one a thread
 constexpr float kMaxWindow = 67108864.0f;   // 2^26 pixels
 
 struct RasterCounters {
     unsigned long long subTris, dropped, pairs, badIdx, badMat;
+    unsigned long long next;   // end of the tile lists laid out so far
+};
+
+struct RasterMats {
+    float model[16], viewProj[16];   // column-major
 };
 
 struct RVert {
@@ -135,14 +140,14 @@ __device__ __forceinline__ void pixel_box(const int *X, const int *Y, int W, int
     y1 = min((mxy - 8) >> 4, H - 1);
 }
 
-__device__ __forceinline__ void store_record(float4 *rec, const SubTri &s, int mat, int valid)
+__device__ __forceinline__ void store_record(float4 *rec, const SubTri &s, int mat)
 {
     rec[0] = make_float4(__int_as_float(s.X[0]), __int_as_float(s.Y[0]), __int_as_float(s.X[1]),
                          __int_as_float(s.Y[1]));
     rec[1] = make_float4(__int_as_float(s.X[2]), __int_as_float(s.Y[2]), __int_as_float((int)(s.area & 0xffffffffll)),
                          __int_as_float((int)(s.area >> 32)));
     rec[2] = make_float4(s.z[0], s.z[1], s.z[2], s.iw[0]);
-    rec[3] = make_float4(s.iw[1], s.iw[2], __int_as_float(mat), __int_as_float(valid));
+    rec[3] = make_float4(s.iw[1], s.iw[2], __int_as_float(mat), 0.0f);
     rec[4] = make_float4(s.p[0][0], s.p[0][1], s.p[0][2], s.p[1][0]);
     rec[5] = make_float4(s.p[1][1], s.p[1][2], s.p[2][0], s.p[2][1]);
     rec[6] = make_float4(s.p[2][2], s.n[0][0], s.n[0][1], s.n[0][2]);
@@ -150,14 +155,21 @@ __device__ __forceinline__ void store_record(float4 *rec, const SubTri &s, int m
     rec[8] = make_float4(s.n[2][1], s.n[2][2], 0.0f, 0.0f);
 }
 
-__device__ __forceinline__ void count_tiles(const SubTri &s, int W, int H, int tilesX, int *tileCount,
-                                            unsigned long long &pairs)
+// First and last tile columns and rows of a sub-triangle's pixel box, 16 bits
+// each; a slot that draws nothing holds (first > last).
+__device__ __forceinline__ uint2 tile_box(const SubTri &s, int W, int H)
 {
     int x0, x1, y0, y1;
     pixel_box(s.X, s.Y, W, H, x0, x1, y0, y1);
-    if (x0 > x1 || y0 > y1) return;
-    for (int ty = y0 / kTile; ty <= y1 / kTile; ++ty)
-        for (int tx = x0 / kTile; tx <= x1 / kTile; ++tx) {
+    if (x0 > x1 || y0 > y1) return make_uint2(1u, 1u);
+    return make_uint2((uint32_t)(x0 / kTile) | (uint32_t)(x1 / kTile) << 16,
+                      (uint32_t)(y0 / kTile) | (uint32_t)(y1 / kTile) << 16);
+}
+
+__device__ __forceinline__ void count_tiles(uint2 b, int tilesX, int *tileCount, unsigned long long &pairs)
+{
+    for (int ty = (int)(b.y & 0xffffu); ty <= (int)(b.y >> 16); ++ty)
+        for (int tx = (int)(b.x & 0xffffu); tx <= (int)(b.x >> 16); ++tx) {
             atomicAdd(&tileCount[ty * tilesX + tx], 1);
             ++pairs;
         }
@@ -172,31 +184,46 @@ __global__ void k_rs_clear(int S, float4 *g0, float4 *g1, float4 *g2, float4 *g3
         g1[p] = q;
         if (g2) g2[p] = q;
         if (g3) g3[p] = q;
-        depth[p] = 1.0f;
+        if (depth) depth[p] = 1.0f;
     }
 }
 
+// The near-plane case (z >= -w, Sutherland-Hodgman), out of line: the polygon's
+// vertices are indexed and would put every triangle's in local memory.
+__device__ __noinline__ int clip_near(const RVert v[3], RVert poly[4])
+{
+    int np = 0;
+    for (int i = 0; i < 3; ++i) {
+        const RVert &a = v[i], &b = v[(i + 1) % 3];
+        const float da = __fadd_rn(a.c[2], a.c[3]), db = __fadd_rn(b.c[2], b.c[3]);
+        if (da >= 0.0f) poly[np++] = a;
+        if ((da >= 0.0f) != (db >= 0.0f)) poly[np++] = lerp_vert(a, b, __fdiv_rn(da, __fsub_rn(da, db)));
+    }
+    return np;
+}
+
+// One thread per triangle.  WIDE: vertices of 32 bytes, 16-byte aligned, with
+// the position first and the normal at float 5 (the MeshManager layout), read
+// as two 16-byte loads.  The counters are summed per block before they reach
+// memory, and a triangle wholly in front of the near plane never touches local
+// memory (1920 x 1080, 331k triangles: 408 -> 27 us).
+template <int WIDE>
 __global__ void __launch_bounds__(128) k_rs_setup(const float *__restrict__ vtx, int V, int strideF, int posOff,
                                                   int nrmOff, const uint32_t *__restrict__ idx, int T,
-                                                  const int32_t *__restrict__ triMat, int nMat, const float *model,
-                                                  const float *viewProj, int W, int H, int tilesX,
-                                                  float4 *__restrict__ recs, int *__restrict__ tileCount,
-                                                  RasterCounters *ctr)
+                                                  const int32_t *__restrict__ triMat, int nMat,
+                                                  const __grid_constant__ RasterMats mats, int W, int H, int tilesX,
+                                                  float4 *__restrict__ recs, uint2 *__restrict__ boxes,
+                                                  int *__restrict__ tileCount, RasterCounters *ctr)
 {
-    __shared__ float sM[16], sVP[16];
-    if (threadIdx.x < 16) {
-        sM[threadIdx.x] = model[threadIdx.x];
-        sVP[threadIdx.x] = viewProj[threadIdx.x];
-    }
+    __shared__ unsigned long long sCount[5];
+    if (threadIdx.x < 5) sCount[threadIdx.x] = 0;
     __syncthreads();
     unsigned long long nsub = 0, ndrop = 0, npairs = 0, nbadI = 0, nbadM = 0;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
         float4 *r0 = recs + (size_t)kRecF4 * (2 * (size_t)t);
-        float4 *r1 = r0 + kRecF4;
-        r0[3].w = __int_as_float(0);
-        r1[3].w = __int_as_float(0);
+        uint2 box0 = make_uint2(1u, 1u), box1 = box0;
         RVert v[3];
-        bool ok = true;
+        bool ok = true, front = true;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             const uint32_t id = idx[3 * (size_t)t + i];
@@ -205,107 +232,128 @@ __global__ void __launch_bounds__(128) k_rs_setup(const float *__restrict__ vtx,
                 break;
             }
             const float *src = vtx + (size_t)id * strideF;
-            const float P[4] = {src[posOff], src[posOff + 1], src[posOff + 2], 1.0f};
-            const float N[4] = {src[nrmOff], src[nrmOff + 1], src[nrmOff + 2], 0.0f};
+            float P[4], N[4];
+            if (WIDE) {
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(src)), b = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+                P[0] = a.x, P[1] = a.y, P[2] = a.z;
+                N[0] = b.y, N[1] = b.z, N[2] = b.w;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    P[k] = src[posOff + k];
+                    N[k] = src[nrmOff + k];
+                }
+            }
+            P[3] = 1.0f;
+            N[3] = 0.0f;
             float wp[4], wn[4];
-            mat_vec4(sM, P, wp);
-            mat_vec4(sM, N, wn);
+            mat_vec4(mats.model, P, wp);
+            mat_vec4(mats.model, N, wn);
             const float WP[4] = {wp[0], wp[1], wp[2], 1.0f};
-            mat_vec4(sVP, WP, v[i].c);
+            mat_vec4(mats.viewProj, WP, v[i].c);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 v[i].p[k] = wp[k];
                 v[i].n[k] = wn[k];
             }
+            front = front && __fadd_rn(v[i].c[2], v[i].c[3]) >= 0.0f;
         }
         if (!ok) {
             ++nbadI;
-            continue;
+        } else {
+            int mat = triMat ? triMat[t] : 0;
+            if (mat < 0 || mat >= nMat) {
+                ++nbadM;
+                mat = 0;
+            }
+            SubTri s;
+            if (front) {
+                const int rc = setup_sub(v[0], v[1], v[2], W, H, s);
+                if (rc == 2) ++ndrop;
+                if (rc == 1) {
+                    store_record(r0, s, mat);
+                    ++nsub;
+                    box0 = tile_box(s, W, H);
+                }
+            } else {
+                RVert in[3] = {v[0], v[1], v[2]}, poly[4];
+                const int np = clip_near(in, poly);
+                for (int k = 0; k < np - 2; ++k) {   // triangle, or quad as two
+                    const int rc = setup_sub(poly[0], poly[k + 1], poly[k + 2], W, H, s);
+                    if (rc == 2) ++ndrop;
+                    if (rc == 1) {
+                        store_record(r0 + k * kRecF4, s, mat);
+                        ++nsub;
+                        (k ? box1 : box0) = tile_box(s, W, H);
+                    }
+                }
+            }
+            count_tiles(box0, tilesX, tileCount, npairs);
+            if (!front) count_tiles(box1, tilesX, tileCount, npairs);
         }
-        int mat = triMat ? triMat[t] : 0;
-        if (mat < 0 || mat >= nMat) {
-            ++nbadM;
-            mat = 0;
-        }
-        // near plane z >= -w (Sutherland-Hodgman)
-        RVert poly[4];
-        int np = 0;
+        reinterpret_cast<uint4 *>(boxes)[t] = make_uint4(box0.x, box0.y, box1.x, box1.y);
+    }
+    unsigned long long c[5] = {nsub, ndrop, npairs, nbadI, nbadM};
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const RVert &a = v[i], &b = v[(i + 1) % 3];
-            const float da = __fadd_rn(a.c[2], a.c[3]), db = __fadd_rn(b.c[2], b.c[3]);
-            if (da >= 0.0f) poly[np++] = a;
-            if ((da >= 0.0f) != (db >= 0.0f)) poly[np++] = lerp_vert(a, b, __fdiv_rn(da, __fsub_rn(da, db)));
-        }
-        SubTri s;
-        if (np >= 3) {
-            const int rc = setup_sub(poly[0], poly[1], poly[2], W, H, s);
-            if (rc == 2) ++ndrop;
-            if (rc == 1) {
-                store_record(r0, s, mat, 1);
-                ++nsub;
-                count_tiles(s, W, H, tilesX, tileCount, npairs);
-            }
-        }
-        if (np == 4) {
-            const int rc = setup_sub(poly[0], poly[2], poly[3], W, H, s);
-            if (rc == 2) ++ndrop;
-            if (rc == 1) {
-                store_record(r1, s, mat, 1);
-                ++nsub;
-                count_tiles(s, W, H, tilesX, tileCount, npairs);
-            }
-        }
+    for (int k = 0; k < 5; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) c[k] += __shfl_xor_sync(kFullWarp, c[k], o);
+        if ((threadIdx.x & 31) == 0 && c[k]) atomicAdd(&sCount[k], c[k]);
     }
-    if (nsub) atomicAdd(&ctr->subTris, nsub);
-    if (ndrop) atomicAdd(&ctr->dropped, ndrop);
-    if (npairs) atomicAdd(&ctr->pairs, npairs);
-    if (nbadI) atomicAdd(&ctr->badIdx, nbadI);
-    if (nbadM) atomicAdd(&ctr->badMat, nbadM);
-}
-
-// Exclusive scan of the tile counts (one block).
-__global__ void __launch_bounds__(1024) k_rs_scan(const int *__restrict__ cnt, int *__restrict__ start, int n)
-{
-    __shared__ long long part[1024];
-    const int per = (n + 1023) / 1024;
-    const int lo = min(n, threadIdx.x * per), hi = min(n, lo + per);
-    long long s = 0;
-    for (int i = lo; i < hi; ++i) s += cnt[i];
-    part[threadIdx.x] = s;
     __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const long long v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    long long run = threadIdx.x ? part[threadIdx.x - 1] : 0;
-    for (int i = lo; i < hi; ++i) {
-        start[i] = (int)run;
-        run += cnt[i];
+    if (threadIdx.x < 5 && sCount[threadIdx.x]) {
+        unsigned long long *dst[5] = {&ctr->subTris, &ctr->dropped, &ctr->pairs, &ctr->badIdx, &ctr->badMat};
+        atomicAdd(dst[threadIdx.x], sCount[threadIdx.x]);
     }
 }
 
-__global__ void k_rs_scatter(const float4 *__restrict__ recs, int slots, int W, int H, int tilesX,
-                             const int *__restrict__ tileStart, int *__restrict__ tileFill, int *__restrict__ pairs,
-                             long long capacity)
+// Lays the tiles' lists out end to end: a block's tiles by a scan of their
+// counts, the blocks in the order in which they arrive (a list's place does not
+// matter; 8,160 tiles: 3 us, 10 us as one block's scan of all tiles).
+__global__ void __launch_bounds__(256) k_rs_lists(const int *__restrict__ cnt, long long *__restrict__ start, int n,
+                                                  RasterCounters *ctr)
 {
-    for (int sl = blockIdx.x * blockDim.x + threadIdx.x; sl < slots; sl += gridDim.x * blockDim.x) {
-        const float4 *r = recs + (size_t)kRecF4 * sl;
-        if (!__float_as_int(r[3].w)) continue;
-        const float4 a = r[0], b = r[1];
-        const int X[3] = {__float_as_int(a.x), __float_as_int(a.z), __float_as_int(b.x)};
-        const int Y[3] = {__float_as_int(a.y), __float_as_int(a.w), __float_as_int(b.y)};
-        int x0, x1, y0, y1;
-        pixel_box(X, Y, W, H, x0, x1, y0, y1);
-        if (x0 > x1 || y0 > y1) continue;
-        for (int ty = y0 / kTile; ty <= y1 / kTile; ++ty)
-            for (int tx = x0 / kTile; tx <= x1 / kTile; ++tx) {
-                const int tile = ty * tilesX + tx;
-                const long long pos = (long long)tileStart[tile] + atomicAdd(&tileFill[tile], 1);
-                if (pos < capacity) pairs[pos] = sl;
-            }
+    __shared__ unsigned long long sWarp[8], sBase;
+    const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned long long c = i < n ? (unsigned long long)cnt[i] : 0ull;
+    unsigned long long x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(kFullWarp, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) sWarp[warp] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long run = 0;
+        for (int k = 0; k < 8; ++k) {
+            const unsigned long long v = sWarp[k];
+            sWarp[k] = run;
+            run += v;
+        }
+        sBase = atomicAdd(&ctr->next, run);
+    }
+    __syncthreads();
+    if (i < n) start[i] = (long long)(sBase + sWarp[warp] + x - c);
+}
+
+__global__ void k_rs_scatter(const uint4 *__restrict__ boxes, int T, int tilesX, const long long *__restrict__ tileStart,
+                             int *__restrict__ tileFill, int *__restrict__ pairs, long long capacity,
+                             const RasterCounters *ctr)
+{
+    if ((long long)ctr->pairs > capacity) return;   // the tiles read the boxes instead
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
+        const uint4 b = boxes[t];
+        auto put = [&](uint32_t bx, uint32_t by, int slot) {
+            for (int ty = (int)(by & 0xffffu); ty <= (int)(by >> 16); ++ty)
+                for (int tx = (int)(bx & 0xffffu); tx <= (int)(bx >> 16); ++tx) {
+                    const int tile = ty * tilesX + tx;
+                    const long long pos = tileStart[tile] + atomicAdd(&tileFill[tile], 1);
+                    if (pos < capacity) pairs[pos] = slot;
+                }
+        };
+        put(b.x, b.y, 2 * t);
+        put(b.z, b.w, 2 * t + 1);
     }
 }
 
@@ -322,65 +370,173 @@ __device__ __forceinline__ long long edge_fn(int ax, int ay, int bx, int by, lon
     return (long long)(bx - ax) * (py - ay) - (long long)(by - ay) * (px - ax);
 }
 
+// A staged record, prepared by one lane for the tile's 256 pixels:
+//  e = edge functions at the tile's first pixel centre, less 1 where a centre on
+//      the edge belongs to the other triangle (bit k of `less`), so that inside
+//      means e >= 0
+//  a, b = their steps per pixel in x and y
+//  z = the vertices' depths, area = twice the area in FP32, rarea its reciprocal
+// In 32 bits for sub-triangles at most 2^14 sixteenths of a pixel across that
+// touch the tile: an edge function within the tile is then below
+// 2 (2^14 + 2^9) 2^14 < 2^30, the exact integer the 64-bit form gives.  Others
+// (and depths beyond 2) have small = 0 and are evaluated from the record.
+struct TileRec {
+    int e[3], slot, a[3], less, b[3], small;
+    float z[3], area;
+    float rarea, pad[3];
+};
+
+// Approximate against exact depth (|z| <= 2): below 2^-19.
+constexpr float kDepthSlack = 1e-5f;
+
+// One block per tile; the tile's list from its buffer or (draws that outgrow
+// it) every slot whose box holds the tile, found by scanning the boxes.  A
+// thread prepares a record, with the warps -- 8 x 4 pixels each -- that have a
+// pixel it can cover (every edge function non-negative at a corner), and each
+// warp goes through its own.  The exact depth (three divisions) is formed
+// only where the approximate one is not clearly behind the pixel's nearest so
+// far.  1920 x 1080, 331k triangles: 705 us as 16 x 2 pixels a warp, every
+// record, 64-bit edge functions.
 __global__ void __launch_bounds__(kTile * kTile) k_rs_tiles(const float4 *__restrict__ recs,
+                                                            const uint2 *__restrict__ boxes, int slots,
                                                             const int *__restrict__ tileCount,
-                                                            const int *__restrict__ tileStart,
+                                                            const long long *__restrict__ tileStart,
                                                             const int *__restrict__ pairs, long long capacity,
-                                                            int W, int H, int tilesX, int clear,
-                                                            const float *__restrict__ mats, float4 *g0, float4 *g1,
-                                                            float4 *g2, float4 *g3, float *depth)
+                                                            const RasterCounters *ctr, int W, int H, int tilesX,
+                                                            int clear, const float *__restrict__ mats, float4 *g0,
+                                                            float4 *g1, float4 *g2, float4 *g3, float *depth)
 {
-    __shared__ float4 s_rec[kChunk][4];   // geometry and depth part of each record
-    __shared__ int s_slot[kChunk];
-    const int tile = blockIdx.x;
+    __shared__ TileRec s_rec[kChunk];
+    __shared__ uint32_t s_warps[kChunk];   // the warps whose pixels a record can touch
+    const int tile = blockIdx.x, tx = tile % tilesX, ty = tile / tilesX;
     const int n = tileCount[tile];
-    if (n == 0) return;
-    const int base = tileStart[tile];
-    const int px = (tile % tilesX) * kTile + (threadIdx.x & (kTile - 1));
-    const int py = (tile / tilesX) * kTile + (threadIdx.x / kTile);
+    if (n == 0 && !clear) return;
+    const bool listed = (long long)ctr->pairs <= capacity;
+    const long long base = tileStart[tile];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wx = 8 * (warp & 1), wy = 4 * (warp >> 1), lx = wx + (lane & 7), ly = wy + (lane >> 3);
+    const int px = tx * kTile + lx, py = ty * kTile + ly;
     const bool inside = px < W && py < H;
     const long long cx = (long long)px * 16 + 8, cy = (long long)py * 16 + 8;
+    const int ox = tx * kTile * 16 + 8, oy = ty * kTile * 16 + 8;   // the tile's first centre
     float bz = __int_as_float(0x7f800000);   // +inf
     int bslot = 0x7fffffff;
-    for (int c0 = 0; c0 < n; c0 += kChunk) {
-        const int m = min(kChunk, n - c0);
+    for (int c0 = 0, scan = 0; c0 < n;) {
         __syncthreads();
-        if (threadIdx.x < m * 4) {
-            const int k = threadIdx.x >> 2, part = threadIdx.x & 3;
-            const long long pi = (long long)base + c0 + k;
-            const int sl = pi < capacity ? pairs[pi] : 0;
-            s_rec[k][part] = recs[(size_t)kRecF4 * sl + part];
-            if (part == 0) s_slot[k] = sl;
+        int sl = -1, m;
+        if (listed) {
+            m = min(kChunk, n - c0);
+            if (threadIdx.x < m) sl = pairs[base + c0 + threadIdx.x];
+        } else {
+            if (scan >= slots) break;
+            bool hit = false;
+            if (scan + lane < slots) {
+                const uint2 b = boxes[scan + lane];
+                hit = tx >= (int)(b.x & 0xffffu) && tx <= (int)(b.x >> 16) && ty >= (int)(b.y & 0xffffu) &&
+                      ty <= (int)(b.y >> 16);
+            }
+            const unsigned hits = __ballot_sync(kFullWarp, hit);
+            m = __popc(hits);
+            if (threadIdx.x < m) sl = scan + (int)__fns(hits, 0, threadIdx.x + 1);
+            scan += 32;
         }
-        __syncthreads();
-        if (!inside) continue;
-        for (int k = 0; k < m; ++k) {
-            const float4 a = s_rec[k][0], b = s_rec[k][1];
-            const int X0 = __float_as_int(a.x), Y0 = __float_as_int(a.y), X1 = __float_as_int(a.z),
-                      Y1 = __float_as_int(a.w), X2 = __float_as_int(b.x), Y2 = __float_as_int(b.y);
-            const long long e0 = edge_fn(X1, Y1, X2, Y2, cx, cy);
-            const long long e1 = edge_fn(X2, Y2, X0, Y0, cx, cy);
-            const long long e2 = edge_fn(X0, Y0, X1, Y1, cx, cy);
-            if (e0 < 0 || e1 < 0 || e2 < 0) continue;
-            if ((e0 == 0 && !edge_owns(X1, Y1, X2, Y2)) || (e1 == 0 && !edge_owns(X2, Y2, X0, Y0)) ||
-                (e2 == 0 && !edge_owns(X0, Y0, X1, Y1)))
-                continue;
+        c0 += m;
+        uint32_t warps = 0;
+        if (sl >= 0) {
+            const float4 *r = recs + (size_t)kRecF4 * sl;
+            const float4 a = __ldg(r), b = __ldg(r + 1), zz = __ldg(r + 2);
+            const int X[3] = {__float_as_int(a.x), __float_as_int(a.z), __float_as_int(b.x)};
+            const int Y[3] = {__float_as_int(a.y), __float_as_int(a.w), __float_as_int(b.y)};
             const long long area = (long long)(unsigned)__float_as_int(b.z) | ((long long)__float_as_int(b.w) << 32);
-            const float fa = __ll2float_rn(area);
-            const float l0 = __fdiv_rn(__ll2float_rn(e0), fa), l1 = __fdiv_rn(__ll2float_rn(e1), fa),
-                        l2 = __fdiv_rn(__ll2float_rn(e2), fa);
-            const float4 zz = s_rec[k][2];
-            const float z = __fadd_rn(__fadd_rn(__fmul_rn(l0, zz.x), __fmul_rn(l1, zz.y)), __fmul_rn(l2, zz.z));
-            if (!(z >= 0.0f && z <= 1.0f)) continue;
-            const int sl = s_slot[k];
-            if (z < bz || (z == bz && sl < bslot)) {
-                bz = z;
-                bslot = sl;
+            const long long wide = (long long)max(X[0], max(X[1], X[2])) - min(X[0], min(X[1], X[2]));
+            const long long high = (long long)max(Y[0], max(Y[1], Y[2])) - min(Y[0], min(Y[1], Y[2]));
+            TileRec &q = s_rec[threadIdx.x];
+            q.slot = sl;
+            q.small = wide <= (1 << 14) && high <= (1 << 14) &&
+                      fmaxf(fmaxf(fabsf(zz.x), fabsf(zz.y)), fabsf(zz.z)) <= 2.0f;
+            q.less = 0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int i = (k + 1) % 3, j = (k + 2) % 3;   // edge k runs from vertex i to vertex j
+                q.e[k] = q.a[k] = q.b[k] = 0;
+                if (q.small) {
+                    const int dx = X[j] - X[i], dy = Y[j] - Y[i], less = edge_owns(X[i], Y[i], X[j], Y[j]) ? 0 : 1;
+                    q.e[k] = dx * (oy - Y[i]) - dy * (ox - X[i]) - less;
+                    q.a[k] = -16 * dy;
+                    q.b[k] = 16 * dx;
+                    q.less |= less << k;
+                }
+            }
+            q.z[0] = zz.x;
+            q.z[1] = zz.y;
+            q.z[2] = zz.z;
+            q.area = __ll2float_rn(area);
+            q.rarea = 1.0f / q.area;
+            // the 8 x 4 pixels of warp w: each edge at the corner where it is largest
+            int e[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) e[k] = q.e[k] + max(7 * q.a[k], 0) + max(3 * q.b[k], 0);
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                const int x = 8 * (w & 1), y = 4 * (w >> 1);
+                int out = 0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) out |= e[k] + q.a[k] * x + q.b[k] * y;
+                if (out >= 0) warps |= 1u << w;
             }
         }
+        s_warps[threadIdx.x] = warps;
+        __syncthreads();
+        for (int first = 0; first < m; first += 32)
+          for (unsigned todo = __ballot_sync(kFullWarp, (s_warps[first + lane] >> warp) & 1u); todo; todo &= todo - 1u) {
+            const TileRec &q = s_rec[first + __ffs(todo) - 1];
+            float f0, f1, f2;
+            if (q.small) {
+                const int e0 = q.e[0] + q.a[0] * lx + q.b[0] * ly, e1 = q.e[1] + q.a[1] * lx + q.b[1] * ly,
+                          e2 = q.e[2] + q.a[2] * lx + q.b[2] * ly;
+                if ((e0 | e1 | e2) < 0 || !inside) continue;
+                f0 = __int2float_rn(e0 + (q.less & 1));
+                f1 = __int2float_rn(e1 + ((q.less >> 1) & 1));
+                f2 = __int2float_rn(e2 + (q.less >> 2));
+                if (((f0 * q.z[0] + f1 * q.z[1]) + f2 * q.z[2]) * q.rarea > bz + kDepthSlack) continue;
+            } else {
+                if (!inside) continue;
+                const float4 *r = recs + (size_t)kRecF4 * q.slot;
+                const float4 a = __ldg(r), b = __ldg(r + 1);
+                const int X0 = __float_as_int(a.x), Y0 = __float_as_int(a.y), X1 = __float_as_int(a.z),
+                          Y1 = __float_as_int(a.w), X2 = __float_as_int(b.x), Y2 = __float_as_int(b.y);
+                const long long e0 = edge_fn(X1, Y1, X2, Y2, cx, cy), e1 = edge_fn(X2, Y2, X0, Y0, cx, cy),
+                                e2 = edge_fn(X0, Y0, X1, Y1, cx, cy);
+                if (e0 < 0 || e1 < 0 || e2 < 0) continue;
+                if ((e0 == 0 && !edge_owns(X1, Y1, X2, Y2)) || (e1 == 0 && !edge_owns(X2, Y2, X0, Y0)) ||
+                    (e2 == 0 && !edge_owns(X0, Y0, X1, Y1)))
+                    continue;
+                f0 = __ll2float_rn(e0);
+                f1 = __ll2float_rn(e1);
+                f2 = __ll2float_rn(e2);
+            }
+            const float l0 = __fdiv_rn(f0, q.area), l1 = __fdiv_rn(f1, q.area), l2 = __fdiv_rn(f2, q.area);
+            const float z = __fadd_rn(__fadd_rn(__fmul_rn(l0, q.z[0]), __fmul_rn(l1, q.z[1])), __fmul_rn(l2, q.z[2]));
+            if (!(z >= 0.0f && z <= 1.0f)) continue;
+            if (z < bz || (z == bz && q.slot < bslot)) {
+                bz = z;
+                bslot = q.slot;
+            }
+          }
     }
-    if (!inside || bslot == 0x7fffffff) return;
+    if (!inside) return;
     const size_t p = (size_t)py * W + px;
+    if (bslot == 0x7fffffff) {
+        if (!clear) return;
+        const float nan = __int_as_float(0x7fc00000);
+        const float4 none = make_float4(nan, nan, nan, nan);
+        g0[p] = none;
+        g1[p] = none;
+        if (g2) g2[p] = none;
+        if (g3) g3[p] = none;
+        if (depth) depth[p] = 1.0f;
+        return;
+    }
     if (!clear && !(bz < depth[p])) return;   // GL_LESS against earlier draws
     const float4 *r = recs + (size_t)kRecF4 * bslot;
     const float4 a = r[0], b = r[1], r2 = r[2], r3 = r[3], r4 = r[4], r5 = r[5], r6 = r[6], r7 = r[7], r8 = r[8];
@@ -404,7 +560,7 @@ __global__ void __launch_bounds__(kTile * kTile) k_rs_tiles(const float4 *__rest
         N[k] = __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(q0, N0[k]), __fmul_rn(q1, N1[k])), __fmul_rn(q2, N2[k])), d);
     }
     const float *mt = mats + 10 * (size_t)__float_as_int(r3.z);
-    depth[p] = bz;
+    if (depth) depth[p] = bz;
     g0[p] = make_float4(P[0], P[1], P[2], mt[6]);
     g1[p] = make_float4(N[0], N[1], N[2], mt[7]);
     if (g2) g2[p] = make_float4(mt[0], mt[1], mt[2], mt[8]);
@@ -421,21 +577,22 @@ static_assert(sizeof(fdzb_raster_desc) == 240, "fdzb_raster_desc layout");
 static_assert(sizeof(fdzb_raster_stats) == 64, "fdzb_raster_stats layout");
 
 struct fdzb_raster {
-    int device = 0;
+    int device = 0, sms = 148;
     cudaStream_t own = nullptr, stream = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     float4 *recs = nullptr;
-    size_t recSlots = 0;
-    int *tileCount = nullptr, *tileStart = nullptr, *tileFill = nullptr;
+    uint2 *boxes = nullptr;
+    size_t recSlots = 0, boxSlots = 0;
+    // counters, then tileCount, tileFill (both cleared with them) and tileStart
+    char *tiles = nullptr;
     size_t tileCap = 0;
     int *pairs = nullptr;
-    long long pairCap = 0;
-    float *depthScratch = nullptr;
-    size_t depthCap = 0;
-    float *dMats = nullptr;   // model and view_proj
-    fdzb::RasterCounters *ctr = nullptr, *hCtr = nullptr;
+    size_t pairCap = 0;
+    unsigned long long lastPairs = 0;
+    fdzb::RasterCounters *hCtr = nullptr;
     fdzb_raster_stats stats{};
     bool pending = false;
+    bool tooMany = false;   // the last draw had more than 2^31 tile pairs
 };
 
 namespace {
@@ -464,16 +621,30 @@ int grow(void **p, size_t &cap, size_t need, size_t elem)
     return FDZB_OK;
 }
 
+constexpr size_t kCtrBytes = 256;
+static_assert(sizeof(fdzb::RasterCounters) <= kCtrBytes, "counters' place before the tile arrays");
+
+// Waits for the draw in flight and takes its counters.
 int finish(fdzb_raster *r)
 {
     if (!r->pending) return FDZB_OK;
     RS_CUDA(cudaEventSynchronize(r->e1));
+    r->pending = false;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, r->e0, r->e1);
+    const fdzb::RasterCounters &c = *r->hCtr;
+    r->lastPairs = c.pairs;
     r->stats.ms = ms;
-    r->pending = false;
+    r->stats.sub_triangles = (int64_t)c.subTris;
+    r->stats.dropped = (int64_t)c.dropped;
+    r->stats.tile_pairs = (int64_t)c.pairs;
+    r->stats.bad_indices = (int64_t)c.badIdx;
+    r->stats.bad_materials = (int64_t)c.badMat;
+    r->tooMany = c.pairs > 0x7fffffffull;
     return FDZB_OK;
 }
+
+int too_many() { return rfail(FDZB_ERR_CAPACITY, "more than 2^31 tile pairs in one draw"); }
 
 }  // namespace
 
@@ -490,13 +661,12 @@ int fdzb_raster_create(fdzb_raster **out, int device)
     r->device = dev;
     if (cudaStreamCreateWithFlags(&r->own, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&r->e0) != cudaSuccess || cudaEventCreate(&r->e1) != cudaSuccess ||
-        cudaMalloc(&r->dMats, 32 * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&r->ctr, sizeof(fdzb::RasterCounters)) != cudaSuccess ||
         cudaMallocHost(&r->hCtr, sizeof(fdzb::RasterCounters)) != cudaSuccess) {
         cudaGetLastError();
         fdzb_raster_destroy(r);
         return rfail(FDZB_ERR_CUDA, "could not create the rasteriser's stream, events or buffers");
     }
+    cudaDeviceGetAttribute(&r->sms, cudaDevAttrMultiProcessorCount, dev);
     r->stream = r->own;
     *out = r;
     return FDZB_OK;
@@ -508,13 +678,9 @@ int fdzb_raster_destroy(fdzb_raster *r)
     cudaSetDevice(r->device);
     if (r->stream) cudaStreamSynchronize(r->stream);
     cudaFree(r->recs);
-    cudaFree(r->tileCount);
-    cudaFree(r->tileStart);
-    cudaFree(r->tileFill);
+    cudaFree(r->boxes);
+    cudaFree(r->tiles);
     cudaFree(r->pairs);
-    cudaFree(r->depthScratch);
-    cudaFree(r->dMats);
-    cudaFree(r->ctr);
     if (r->hCtr) cudaFreeHost(r->hCtr);
     if (r->e0) cudaEventDestroy(r->e0);
     if (r->e1) cudaEventDestroy(r->e1);
@@ -535,7 +701,8 @@ int fdzb_raster_sync(fdzb_raster *r)
 {
     if (!r) return rfail(FDZB_ERR_INVALID_ARG, "handle is NULL");
     cudaSetDevice(r->device);
-    return finish(r);
+    if (int rc = finish(r)) return rc;
+    return r->tooMany ? too_many() : FDZB_OK;
 }
 
 int fdzb_raster_get_stats(fdzb_raster *r, fdzb_raster_stats *st)
@@ -570,78 +737,67 @@ int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *d)
     const size_t S = (size_t)W * H;
     const int tilesX = (W + 15) / 16, tilesY = (H + 15) / 16;
     const size_t nTiles = (size_t)tilesX * tilesY;
-    float *depth = d->d_depth;
-    if (!depth) {
-        if (int rc = grow((void **)&r->depthScratch, r->depthCap, S, sizeof(float))) return rc;
-        depth = r->depthScratch;
-    }
-    if (int rc = grow((void **)&r->recs, r->recSlots, 2 * (size_t)std::max(d->n_tri, 1), kRecF4 * sizeof(float4))) return rc;
+    const size_t T = (size_t)d->n_tri;
+    if (int rc = grow((void **)&r->recs, r->recSlots, 2 * std::max<size_t>(T, 1), kRecF4 * sizeof(float4))) return rc;
+    if (int rc = grow((void **)&r->boxes, r->boxSlots, 2 * std::max<size_t>(T, 1), sizeof(uint2))) return rc;
+    // tileCount, tileFill and tileStart of a capacity of r->tileCap tiles
     if (nTiles > r->tileCap) {
-        // the three per-tile arrays share one capacity
-        cudaFree(r->tileCount);
-        cudaFree(r->tileStart);
-        cudaFree(r->tileFill);
-        r->tileCount = r->tileStart = r->tileFill = nullptr;
+        size_t bytes = 0;
+        const size_t cap = (nTiles + nTiles / 4 + 64) / 2 * 2;
+        cudaFree(r->tiles);
+        r->tiles = nullptr;
         r->tileCap = 0;
-        const size_t cap = nTiles + nTiles / 4 + 64;
-        if (cudaMalloc(&r->tileCount, cap * sizeof(int)) != cudaSuccess ||
-            cudaMalloc(&r->tileStart, cap * sizeof(int)) != cudaSuccess ||
-            cudaMalloc(&r->tileFill, cap * sizeof(int)) != cudaSuccess) {
-            cudaGetLastError();
-            return rfail(FDZB_ERR_NO_MEMORY, "device allocation failed");
-        }
+        if (int rc = grow((void **)&r->tiles, bytes, kCtrBytes + cap * 16, 1)) return rc;
         r->tileCap = cap;
     }
+    // the tile lists: from the triangles and tiles, or a quarter more than the last draw's
+    const size_t want = std::min<size_t>(std::max<size_t>(6 * T + 4 * nTiles, (size_t)r->lastPairs + (size_t)r->lastPairs / 4), 0x7fffffffull);
+    if (T > 0)
+        if (int rc = grow((void **)&r->pairs, r->pairCap, want, sizeof(int))) return rc;
+    RasterCounters *ctr = (RasterCounters *)r->tiles;
+    int *tileCount = (int *)(r->tiles + kCtrBytes), *tileFill = tileCount + nTiles;
+    long long *tileStart = (long long *)(r->tiles + kCtrBytes + 8 * nTiles);
     cudaStream_t s = r->stream;
-    int sm = 148;
-    cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, r->device);
-    float mats[32];
-    std::memcpy(mats, d->model, sizeof(d->model));
-    std::memcpy(mats + 16, d->view_proj, sizeof(d->view_proj));
+    const int sm = r->sms;
+    RasterMats mats;
+    std::memcpy(mats.model, d->model, sizeof(mats.model));
+    std::memcpy(mats.viewProj, d->view_proj, sizeof(mats.viewProj));
     RS_CUDA(cudaEventRecord(r->e0, s));
-    RS_CUDA(cudaMemcpyAsync(r->dMats, mats, sizeof(mats), cudaMemcpyHostToDevice, s));
-    RS_CUDA(cudaMemsetAsync(r->ctr, 0, sizeof(RasterCounters), s));
-    RS_CUDA(cudaMemsetAsync(r->tileCount, 0, nTiles * sizeof(int), s));
-    RS_CUDA(cudaMemsetAsync(r->tileFill, 0, nTiles * sizeof(int), s));
-    if (d->clear) {
+    RS_CUDA(cudaMemsetAsync(r->tiles, 0, kCtrBytes + 8 * nTiles, s));
+    if (T > 0) {
+        const int g = (int)std::min<long long>((d->n_tri + 127) / 128, (long long)sm * 16);
+        const bool wide = strideF == 8 && d->pos_offset == 0 && d->nrm_offset == 5 && !((uintptr_t)d->d_vtx & 15);
+        auto setup = wide ? k_rs_setup<1> : k_rs_setup<0>;
+        setup<<<g, 128, 0, s>>>(d->d_vtx, d->n_vtx, strideF, d->pos_offset, d->nrm_offset, d->d_idx, d->n_tri,
+                                d->d_tri_material, d->n_materials, mats, W, H, tilesX, r->recs, r->boxes, tileCount, ctr);
+        k_rs_lists<<<(unsigned)((nTiles + 255) / 256), 256, 0, s>>>(tileCount, tileStart, (int)nTiles, ctr);
+        // A draw whose lists outgrow their buffer scans the slots' boxes, slots / 32
+        // rounds a tile: where that could take long (2^36 slots x tiles: about 0.2
+        // s), the host waits for the lists' size instead and makes the buffer fit.
+        if (2ull * T * nTiles > (1ull << 36)) {
+            RS_CUDA(cudaMemcpyAsync(r->hCtr, ctr, sizeof(RasterCounters), cudaMemcpyDeviceToHost, s));
+            RS_CUDA(cudaStreamSynchronize(s));
+            if (r->hCtr->pairs > 0x7fffffffull) return too_many();
+            if (int rc = grow((void **)&r->pairs, r->pairCap, (size_t)r->hCtr->pairs, sizeof(int))) return rc;
+        }
+        k_rs_scatter<<<(int)std::min<long long>((d->n_tri + 255) / 256, (long long)sm * 8), 256, 0, s>>>(
+            (const uint4 *)r->boxes, d->n_tri, tilesX, tileStart, tileFill, r->pairs, (long long)r->pairCap, ctr);
+        k_rs_tiles<<<(unsigned)nTiles, 256, 0, s>>>(r->recs, r->boxes, 2 * d->n_tri, tileCount, tileStart, r->pairs,
+                                                    (long long)r->pairCap, ctr, W, H, tilesX, d->clear, d->d_materials,
+                                                    (float4 *)d->d_g0, (float4 *)d->d_g1, (float4 *)d->d_g2,
+                                                    (float4 *)d->d_g3, d->d_depth);
+    } else if (d->clear) {
         const int g = (int)std::min<size_t>((S + 255) / 256, (size_t)sm * 8);
         k_rs_clear<<<g, 256, 0, s>>>((int)S, (float4 *)d->d_g0, (float4 *)d->d_g1, (float4 *)d->d_g2,
-                                     (float4 *)d->d_g3, depth);
-    }
-    if (d->n_tri > 0) {
-        const int g = (int)std::min<long long>((d->n_tri + 127) / 128, (long long)sm * 16);
-        k_rs_setup<<<g, 128, 0, s>>>(d->d_vtx, d->n_vtx, strideF, d->pos_offset, d->nrm_offset, d->d_idx, d->n_tri,
-                                     d->d_tri_material, d->n_materials, r->dMats, r->dMats + 16, W, H, tilesX,
-                                     r->recs, r->tileCount, r->ctr);
-        k_rs_scan<<<1, 1024, 0, s>>>(r->tileCount, r->tileStart, (int)nTiles);
+                                     (float4 *)d->d_g3, d->d_depth);
     }
     RS_CUDA(cudaGetLastError());
-    RS_CUDA(cudaMemcpyAsync(r->hCtr, r->ctr, sizeof(RasterCounters), cudaMemcpyDeviceToHost, s));
-    RS_CUDA(cudaStreamSynchronize(s));
-    const RasterCounters c = *r->hCtr;
+    RS_CUDA(cudaMemcpyAsync(r->hCtr, ctr, sizeof(RasterCounters), cudaMemcpyDeviceToHost, s));
+    RS_CUDA(cudaEventRecord(r->e1, s));
     r->stats = fdzb_raster_stats{};
     r->stats.triangles = d->n_tri;
-    r->stats.sub_triangles = (int64_t)c.subTris;
-    r->stats.dropped = (int64_t)c.dropped;
-    r->stats.tile_pairs = (int64_t)c.pairs;
-    r->stats.bad_indices = (int64_t)c.badIdx;
-    r->stats.bad_materials = (int64_t)c.badMat;
     r->stats.tiles_x = tilesX;
     r->stats.tiles_y = tilesY;
-    if (c.pairs > (unsigned long long)0x7fffffff) return rfail(FDZB_ERR_CAPACITY, "more than 2^31 tile pairs in one draw");
-    if (d->n_tri > 0 && c.pairs > 0) {
-        size_t pc = (size_t)r->pairCap;
-        if (int rc = grow((void **)&r->pairs, pc, (size_t)c.pairs, sizeof(int))) return rc;
-        r->pairCap = (long long)pc;
-        const int slots = 2 * d->n_tri;
-        const int g = (int)std::min<long long>((slots + 255) / 256, (long long)sm * 16);
-        k_rs_scatter<<<g, 256, 0, s>>>(r->recs, slots, W, H, tilesX, r->tileStart, r->tileFill, r->pairs, r->pairCap);
-        k_rs_tiles<<<(unsigned)nTiles, 256, 0, s>>>(r->recs, r->tileCount, r->tileStart, r->pairs, r->pairCap, W, H,
-                                                    tilesX, d->clear, d->d_materials, (float4 *)d->d_g0,
-                                                    (float4 *)d->d_g1, (float4 *)d->d_g2, (float4 *)d->d_g3, depth);
-        RS_CUDA(cudaGetLastError());
-    }
-    RS_CUDA(cudaEventRecord(r->e1, s));
     r->pending = true;
     return FDZB_OK;
 }

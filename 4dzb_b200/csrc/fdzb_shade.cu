@@ -25,16 +25,23 @@ __device__ __forceinline__ float3 f3n(float3 v)
     return make_float3(v.x * r, v.y * r, v.z * r);
 }
 
-__global__ void __launch_bounds__(256) k_shade(int npix, const float4 *__restrict__ g0,
+// ONE: a single light sample, as the application shades with: HBM-bound, so 8
+// blocks an SM with all five of a pixel's loads in flight (1920 x 1080: 39 -> 26
+// us, 6.6 TB/s; 6 blocks 34 us).  More samples: ALU-bound (the powers), where the
+// 40 registers of 6 blocks are the faster form (64 samples: 559 us, 639 at 8).
+template <int ONE>
+__global__ void __launch_bounds__(256, ONE ? 8 : 6) k_shade(int npix, const float4 *__restrict__ g0,
                                                const float4 *__restrict__ g1, const float4 *__restrict__ g2,
                                                const float4 *__restrict__ g3, const float *__restrict__ shadow,
                                                float4 *__restrict__ out, float3 cam, float3 La, float3 Ld,
                                                float3 Ls, const float *__restrict__ lights, int nl)
 {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
-        const float I = 1.0f - shadow[p];
+        // all five loads in flight before the shadow value decides
+        const float sh = __ldcs(shadow + p);
+        const float4 a = __ldcs(g0 + p), b = __ldcs(g1 + p), c = __ldcs(g2 + p), d = __ldcs(g3 + p);
+        const float I = 1.0f - sh;
         if (isnan(I)) continue;
-        const float4 a = g0[p], b = g1[p], c = g2[p], d = g3[p];
         const float3 wp = make_float3(a.x, a.y, a.z);
         const float3 N = f3n(make_float3(b.x, b.y, b.z));
         const float3 ka = make_float3(c.x, c.y, c.z), kd = make_float3(d.x, d.y, d.z);
@@ -43,7 +50,8 @@ __global__ void __launch_bounds__(256) k_shade(int npix, const float4 *__restric
         const float3 V = f3n(make_float3(cam.x - wp.x, cam.y - wp.y, cam.z - wp.z));
         const float3 amb = make_float3(La.x * ka.x, La.y * ka.y, La.z * ka.z);
         float3 acc = make_float3(0.f, 0.f, 0.f);
-        for (int i = 0; i < nl; ++i) {
+        const int count = ONE ? 1 : nl;
+        for (int i = 0; i < count; ++i) {
             const float3 lp = make_float3(__ldg(lights + 3 * i), __ldg(lights + 3 * i + 1), __ldg(lights + 3 * i + 2));
             const float3 L = f3n(make_float3(lp.x - wp.x, lp.y - wp.y, lp.z - wp.z));
             const float ldn = L.x * N.x + L.y * N.y + L.z * N.z;
@@ -54,7 +62,7 @@ __global__ void __launch_bounds__(256) k_shade(int npix, const float4 *__restric
             acc.y += amb.y + (Ld.y * kd.y * dif + Ls.y * ks.y * spec) * I;
             acc.z += amb.z + (Ld.z * kd.z * dif + Ls.z * ks.z * spec) * I;
         }
-        const float inv = 1.0f / (float)nl;
+        const float inv = 1.0f / (float)count;
         out[p] = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, 1.0f);
     }
 }
@@ -81,7 +89,8 @@ extern "C" int fdzb_shade(const fdzb_shade_desc *d, void *stream)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     long long g = (npix + 255) / 256;
     const int grid = (int)(g > (long long)sms * 8 ? (long long)sms * 8 : (g < 1 ? 1 : g));
-    k_shade<<<grid, 256, 0, (cudaStream_t)stream>>>(
+    auto kernel = d->n_light_samples == 1 ? k_shade<1> : k_shade<0>;
+    kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
         npix, (const float4 *)d->d_g0, (const float4 *)d->d_g1, (const float4 *)d->d_g2, (const float4 *)d->d_g3,
         d->d_shadow, (float4 *)d->d_rgba, make_float3(d->camera_pos[0], d->camera_pos[1], d->camera_pos[2]),
         make_float3(d->La[0], d->La[1], d->La[2]), make_float3(d->Ld[0], d->Ld[1], d->Ld[2]),
