@@ -166,13 +166,43 @@ __device__ __forceinline__ uint2 tile_box(const SubTri &s, int W, int H)
                       (uint32_t)(y0 / kTile) | (uint32_t)(y1 / kTile) << 16);
 }
 
-__device__ __forceinline__ void count_tiles(uint2 b, int tilesX, int *tileCount, unsigned long long &pairs)
+__device__ __forceinline__ int box_tiles(uint2 b)
 {
-    for (int ty = (int)(b.y & 0xffffu); ty <= (int)(b.y >> 16); ++ty)
-        for (int tx = (int)(b.x & 0xffffu); tx <= (int)(b.x >> 16); ++tx) {
-            atomicAdd(&tileCount[ty * tilesX + tx], 1);
-            ++pairs;
+    const int w = (int)(b.x >> 16) - (int)(b.x & 0xffffu) + 1;
+    return w > 0 ? w * ((int)(b.y >> 16) - (int)(b.y & 0xffffu) + 1) : 0;
+}
+
+// Calls f(k, tile) for tiles first..first + 3 of a box, row by row.
+template <class F> __device__ __forceinline__ void four_tiles(uint2 b, int first, int n, int tilesX, F f)
+{
+    const int x0 = (int)(b.x & 0xffffu), w = (int)(b.x >> 16) - x0 + 1, y0 = (int)(b.y & 0xffffu);
+    int y = first / w, x = first - y * w;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (first + k < n) f(k, (y0 + y) * tilesX + x0 + x);
+        if (++x == w) {
+            x = 0;
+            ++y;
         }
+    }
+}
+
+// Counts a slot's tiles.  The tiles of a box of at most four (most of them) are
+// counted with their answer, the slot's place in the tile's list, which saves
+// the scatter its own atomics; larger boxes only raise the tile's second count.
+__device__ __forceinline__ void count_tiles(uint2 b, int tilesX, int *tileCount, int *tileMore, uint4 *__restrict__ place,
+                                            unsigned long long &pairs)
+{
+    const int n = box_tiles(b);
+    pairs += (unsigned long long)n;
+    if (n > 4) {
+        for (int k0 = 0; k0 < n; k0 += 4)
+            four_tiles(b, k0, n, tilesX, [&](int, int tile) { atomicAdd(&tileMore[tile], 1); });
+    } else if (n > 0) {
+        uint32_t at[4] = {0u, 0u, 0u, 0u};
+        four_tiles(b, 0, n, tilesX, [&](int k, int tile) { at[k] = (uint32_t)atomicAdd(&tileCount[tile], 1); });
+        *place = make_uint4(at[0], at[1], at[2], at[3]);
+    }
 }
 
 __global__ void k_rs_clear(int S, float4 *g0, float4 *g1, float4 *g2, float4 *g3, float *depth)
@@ -206,14 +236,16 @@ __device__ __noinline__ int clip_near(const RVert v[3], RVert poly[4])
 // the position first and the normal at float 5 (the MeshManager layout), read
 // as two 16-byte loads.  The counters are summed per block before they reach
 // memory, and a triangle wholly in front of the near plane never touches local
-// memory (1920 x 1080, 331k triangles: 408 -> 27 us).
+// memory (1920 x 1080, 331k triangles: 408 -> 47 us; bound by the scattered
+// vertex reads and the tile counts' atomics).
 template <int WIDE>
 __global__ void __launch_bounds__(128) k_rs_setup(const float *__restrict__ vtx, int V, int strideF, int posOff,
                                                   int nrmOff, const uint32_t *__restrict__ idx, int T,
                                                   const int32_t *__restrict__ triMat, int nMat,
                                                   const __grid_constant__ RasterMats mats, int W, int H, int tilesX,
                                                   float4 *__restrict__ recs, uint2 *__restrict__ boxes,
-                                                  int *__restrict__ tileCount, RasterCounters *ctr)
+                                                  uint4 *__restrict__ places, int *__restrict__ tileCount,
+                                                  int *__restrict__ tileMore, RasterCounters *ctr)
 {
     __shared__ unsigned long long sCount[5];
     if (threadIdx.x < 5) sCount[threadIdx.x] = 0;
@@ -288,8 +320,8 @@ __global__ void __launch_bounds__(128) k_rs_setup(const float *__restrict__ vtx,
                     }
                 }
             }
-            count_tiles(box0, tilesX, tileCount, npairs);
-            if (!front) count_tiles(box1, tilesX, tileCount, npairs);
+            count_tiles(box0, tilesX, tileCount, tileMore, places + 2 * (size_t)t, npairs);
+            if (!front) count_tiles(box1, tilesX, tileCount, tileMore, places + 2 * (size_t)t + 1, npairs);
         }
         reinterpret_cast<uint4 *>(boxes)[t] = make_uint4(box0.x, box0.y, box1.x, box1.y);
     }
@@ -310,12 +342,12 @@ __global__ void __launch_bounds__(128) k_rs_setup(const float *__restrict__ vtx,
 // Lays the tiles' lists out end to end: a block's tiles by a scan of their
 // counts, the blocks in the order in which they arrive (a list's place does not
 // matter; 8,160 tiles: 3 us, 10 us as one block's scan of all tiles).
-__global__ void __launch_bounds__(256) k_rs_lists(const int *__restrict__ cnt, long long *__restrict__ start, int n,
-                                                  RasterCounters *ctr)
+__global__ void __launch_bounds__(256) k_rs_lists(const int *__restrict__ cnt, const int *__restrict__ more,
+                                                  long long *__restrict__ start, int n, RasterCounters *ctr)
 {
     __shared__ unsigned long long sWarp[8], sBase;
     const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned long long c = i < n ? (unsigned long long)cnt[i] : 0ull;
+    const unsigned long long c = i < n ? (unsigned long long)cnt[i] + (unsigned long long)more[i] : 0ull;
     unsigned long long x = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -337,23 +369,40 @@ __global__ void __launch_bounds__(256) k_rs_lists(const int *__restrict__ cnt, l
     if (i < n) start[i] = (long long)(sBase + sWarp[warp] + x - c);
 }
 
-__global__ void k_rs_scatter(const uint4 *__restrict__ boxes, int T, int tilesX, const long long *__restrict__ tileStart,
+__global__ void k_rs_scatter(const uint4 *__restrict__ boxes, const uint4 *__restrict__ places, int T, int tilesX,
+                             const int *__restrict__ tileCount, const long long *__restrict__ tileStart,
                              int *__restrict__ tileFill, int *__restrict__ pairs, long long capacity,
                              const RasterCounters *ctr)
 {
     if ((long long)ctr->pairs > capacity) return;   // the tiles read the boxes instead
+    auto put = [&](uint2 b, int slot) {
+        const int n = box_tiles(b);
+        if (n > 4) {
+            // after the tile's counted places, by an atomic; four at a time, since
+            // an atomic's answer takes longer than everything else here
+            for (int k0 = 0; k0 < n; k0 += 4) {
+                long long at[4] = {-1, -1, -1, -1};
+                four_tiles(b, k0, n, tilesX, [&](int k, int tile) {
+                    at[k] = tileStart[tile] + tileCount[tile] + atomicAdd(&tileFill[tile], 1);
+                });
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (at[k] >= 0 && at[k] < capacity) pairs[at[k]] = slot;
+            }
+        } else if (n > 0) {
+            const uint4 q = places[slot];
+            const uint32_t in[4] = {q.x, q.y, q.z, q.w};
+            long long at[4] = {-1, -1, -1, -1};
+            four_tiles(b, 0, n, tilesX, [&](int k, int tile) { at[k] = tileStart[tile] + in[k]; });
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (at[k] >= 0 && at[k] < capacity) pairs[at[k]] = slot;
+        }
+    };
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
         const uint4 b = boxes[t];
-        auto put = [&](uint32_t bx, uint32_t by, int slot) {
-            for (int ty = (int)(by & 0xffffu); ty <= (int)(by >> 16); ++ty)
-                for (int tx = (int)(bx & 0xffffu); tx <= (int)(bx >> 16); ++tx) {
-                    const int tile = ty * tilesX + tx;
-                    const long long pos = tileStart[tile] + atomicAdd(&tileFill[tile], 1);
-                    if (pos < capacity) pairs[pos] = slot;
-                }
-        };
-        put(b.x, b.y, 2 * t);
-        put(b.z, b.w, 2 * t + 1);
+        put(make_uint2(b.x, b.y), 2 * t);
+        put(make_uint2(b.z, b.w), 2 * t + 1);
     }
 }
 
@@ -396,10 +445,11 @@ constexpr float kDepthSlack = 1e-5f;
 // warp goes through its own.  The exact depth (three divisions) is formed
 // only where the approximate one is not clearly behind the pixel's nearest so
 // far.  1920 x 1080, 331k triangles: 705 us as 16 x 2 pixels a warp, every
-// record, 64-bit edge functions.
+// record, 64-bit edge functions; 170 us in this form (70 % of issue slots busy).
 __global__ void __launch_bounds__(kTile * kTile) k_rs_tiles(const float4 *__restrict__ recs,
                                                             const uint2 *__restrict__ boxes, int slots,
                                                             const int *__restrict__ tileCount,
+                                                            const int *__restrict__ tileMore,
                                                             const long long *__restrict__ tileStart,
                                                             const int *__restrict__ pairs, long long capacity,
                                                             const RasterCounters *ctr, int W, int H, int tilesX,
@@ -409,7 +459,7 @@ __global__ void __launch_bounds__(kTile * kTile) k_rs_tiles(const float4 *__rest
     __shared__ TileRec s_rec[kChunk];
     __shared__ uint32_t s_warps[kChunk];   // the warps whose pixels a record can touch
     const int tile = blockIdx.x, tx = tile % tilesX, ty = tile / tilesX;
-    const int n = tileCount[tile];
+    const int n = tileCount[tile] + tileMore[tile];
     if (n == 0 && !clear) return;
     const bool listed = (long long)ctr->pairs <= capacity;
     const long long base = tileStart[tile];
@@ -582,8 +632,9 @@ struct fdzb_raster {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     float4 *recs = nullptr;
     uint2 *boxes = nullptr;
-    size_t recSlots = 0, boxSlots = 0;
-    // counters, then tileCount, tileFill (both cleared with them) and tileStart
+    uint4 *places = nullptr;
+    size_t recSlots = 0, boxSlots = 0, placeSlots = 0;
+    // counters, then tileCount, tileMore, tileFill (cleared with them) and tileStart
     char *tiles = nullptr;
     size_t tileCap = 0;
     int *pairs = nullptr;
@@ -679,6 +730,7 @@ int fdzb_raster_destroy(fdzb_raster *r)
     if (r->stream) cudaStreamSynchronize(r->stream);
     cudaFree(r->recs);
     cudaFree(r->boxes);
+    cudaFree(r->places);
     cudaFree(r->tiles);
     cudaFree(r->pairs);
     if (r->hCtr) cudaFreeHost(r->hCtr);
@@ -740,14 +792,15 @@ int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *d)
     const size_t T = (size_t)d->n_tri;
     if (int rc = grow((void **)&r->recs, r->recSlots, 2 * std::max<size_t>(T, 1), kRecF4 * sizeof(float4))) return rc;
     if (int rc = grow((void **)&r->boxes, r->boxSlots, 2 * std::max<size_t>(T, 1), sizeof(uint2))) return rc;
-    // tileCount, tileFill and tileStart of a capacity of r->tileCap tiles
+    if (int rc = grow((void **)&r->places, r->placeSlots, 2 * std::max<size_t>(T, 1), sizeof(uint4))) return rc;
+    // the four arrays of a capacity of r->tileCap tiles
     if (nTiles > r->tileCap) {
         size_t bytes = 0;
         const size_t cap = (nTiles + nTiles / 4 + 64) / 2 * 2;
         cudaFree(r->tiles);
         r->tiles = nullptr;
         r->tileCap = 0;
-        if (int rc = grow((void **)&r->tiles, bytes, kCtrBytes + cap * 16, 1)) return rc;
+        if (int rc = grow((void **)&r->tiles, bytes, kCtrBytes + cap * 20 + 8, 1)) return rc;
         r->tileCap = cap;
     }
     // the tile lists: from the triangles and tiles, or a quarter more than the last draw's
@@ -755,22 +808,24 @@ int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *d)
     if (T > 0)
         if (int rc = grow((void **)&r->pairs, r->pairCap, want, sizeof(int))) return rc;
     RasterCounters *ctr = (RasterCounters *)r->tiles;
-    int *tileCount = (int *)(r->tiles + kCtrBytes), *tileFill = tileCount + nTiles;
-    long long *tileStart = (long long *)(r->tiles + kCtrBytes + 8 * nTiles);
+    int *tileCount = (int *)(r->tiles + kCtrBytes), *tileMore = tileCount + nTiles, *tileFill = tileMore + nTiles;
+    const size_t cleared = kCtrBytes + (12 * nTiles + 7) / 8 * 8;
+    long long *tileStart = (long long *)(r->tiles + cleared);
     cudaStream_t s = r->stream;
     const int sm = r->sms;
     RasterMats mats;
     std::memcpy(mats.model, d->model, sizeof(mats.model));
     std::memcpy(mats.viewProj, d->view_proj, sizeof(mats.viewProj));
     RS_CUDA(cudaEventRecord(r->e0, s));
-    RS_CUDA(cudaMemsetAsync(r->tiles, 0, kCtrBytes + 8 * nTiles, s));
+    RS_CUDA(cudaMemsetAsync(r->tiles, 0, cleared, s));
     if (T > 0) {
         const int g = (int)std::min<long long>((d->n_tri + 127) / 128, (long long)sm * 16);
         const bool wide = strideF == 8 && d->pos_offset == 0 && d->nrm_offset == 5 && !((uintptr_t)d->d_vtx & 15);
         auto setup = wide ? k_rs_setup<1> : k_rs_setup<0>;
         setup<<<g, 128, 0, s>>>(d->d_vtx, d->n_vtx, strideF, d->pos_offset, d->nrm_offset, d->d_idx, d->n_tri,
-                                d->d_tri_material, d->n_materials, mats, W, H, tilesX, r->recs, r->boxes, tileCount, ctr);
-        k_rs_lists<<<(unsigned)((nTiles + 255) / 256), 256, 0, s>>>(tileCount, tileStart, (int)nTiles, ctr);
+                                d->d_tri_material, d->n_materials, mats, W, H, tilesX, r->recs, r->boxes,
+                                r->places, tileCount, tileMore, ctr);
+        k_rs_lists<<<(unsigned)((nTiles + 255) / 256), 256, 0, s>>>(tileCount, tileMore, tileStart, (int)nTiles, ctr);
         // A draw whose lists outgrow their buffer scans the slots' boxes, slots / 32
         // rounds a tile: where that could take long (2^36 slots x tiles: about 0.2
         // s), the host waits for the lists' size instead and makes the buffer fit.
@@ -781,8 +836,9 @@ int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *d)
             if (int rc = grow((void **)&r->pairs, r->pairCap, (size_t)r->hCtr->pairs, sizeof(int))) return rc;
         }
         k_rs_scatter<<<(int)std::min<long long>((d->n_tri + 255) / 256, (long long)sm * 8), 256, 0, s>>>(
-            (const uint4 *)r->boxes, d->n_tri, tilesX, tileStart, tileFill, r->pairs, (long long)r->pairCap, ctr);
-        k_rs_tiles<<<(unsigned)nTiles, 256, 0, s>>>(r->recs, r->boxes, 2 * d->n_tri, tileCount, tileStart, r->pairs,
+            (const uint4 *)r->boxes, r->places, d->n_tri, tilesX, tileCount, tileStart, tileFill, r->pairs,
+            (long long)r->pairCap, ctr);
+        k_rs_tiles<<<(unsigned)nTiles, 256, 0, s>>>(r->recs, r->boxes, 2 * d->n_tri, tileCount, tileMore, tileStart, r->pairs,
                                                     (long long)r->pairCap, ctr, W, H, tilesX, d->clear, d->d_materials,
                                                     (float4 *)d->d_g0, (float4 *)d->d_g1, (float4 *)d->d_g2,
                                                     (float4 *)d->d_g3, d->d_depth);
