@@ -96,12 +96,13 @@ size_t layout(fdzb::DeviceBuffers &b, char *base, int nf, long long S, long long
     b.totalTris = (int)T;
     b.totalBins = (int)NB;
     b.pairCapacity = (int)P;
+    // two blocks that the host copies whole: frames and bases, counters and states
     b.frames = (fdzb::FrameDesc *)take(sizeof(fdzb::FrameDesc) * nf);
-    b.states = (fdzb::FrameState *)take(sizeof(fdzb::FrameState) * nf);
+    b.sampleBases = (int *)take(sizeof(int) * 3 * nf);
     b.counters = (fdzb::Counters *)take(sizeof(fdzb::Counters));
+    b.states = (fdzb::FrameState *)take(sizeof(fdzb::FrameState) * nf);
     b.epochWord = (uint32_t *)take(sizeof(uint32_t));
     b.sortHist = (uint32_t *)take(sizeof(uint32_t) * 4 * fdzb::kSortSlots * 256);
-    b.sampleBases = (int *)take(sizeof(int) * 3 * nf);
     b.triBases = b.sampleBases ? b.sampleBases + nf : nullptr;
     b.binBases = b.sampleBases ? b.sampleBases + 2 * nf : nullptr;
     const size_t Ss = (size_t)std::max(S, 1ll), Ts = (size_t)std::max(T, 1ll), Ps = (size_t)std::max(P, 1ll);
@@ -126,9 +127,10 @@ size_t layout(fdzb::DeviceBuffers &b, char *base, int nf, long long S, long long
     b.pvalsB = (uint32_t *)take(4 * Ps);
     b.binTriStart = (int32_t *)take(4 * (size_t)NB);
     b.binTriEnd = (int32_t *)take(4 * (size_t)NB);
-    const size_t tiles = (std::max(std::max(Ss, Ps), Ts) + fdzb::kSortTileHost - 1) / fdzb::kSortTileHost;
-    b.sortStatusTiles = tiles;
-    b.sortStatus = (unsigned long long *)take(8 * 256 * tiles);
+    b.sortStatusTiles = (Ps + fdzb::kSortTileHost - 1) / fdzb::kSortTileHost;
+    b.sortStatus = (unsigned long long *)take(8 * 256 * b.sortStatusTiles);
+    b.auxStatusTiles = (std::max(Ss, Ts) + fdzb::kSortTileHost - 1) / fdzb::kSortTileHost;
+    b.auxStatus = (unsigned long long *)take(8 * 256 * b.auxStatusTiles);
     b.itemCapacity = (int)(Ss / 32 + (size_t)NB + (size_t)nf + 1);
     b.items = (int4 *)take(16 * (size_t)b.itemCapacity);
     b.dbgKeys = b.dbgVals = b.dbgPKeys = b.dbgPVals = nullptr;
@@ -180,23 +182,31 @@ int ensure_arena(Engine &e, int nf, long long S, long long T, long long NB, long
     return FDZB_OK;
 }
 
+// Bytes of the frame table and of the counters up to what lies behind them.
+size_t frames_bytes(int nf) { return align_up(sizeof(fdzb::FrameDesc) * (size_t)nf, 256); }
+constexpr size_t kCountersBytes = (sizeof(fdzb::Counters) + 255) / 256 * 256;
+
 int ensure_host(Engine &e, int nf)
 {
+    e.hBases = (int *)((char *)e.hFrames + frames_bytes(nf));
     if (nf <= e.hCap) return FDZB_OK;
     if (e.pending) cudaStreamSynchronize(e.stream);
     drop_graph(e);
     if (e.hFrames) cudaFreeHost(e.hFrames);
-    if (e.hStates) cudaFreeHost(e.hStates);
-    if (e.hBases) cudaFreeHost(e.hBases);
+    fdzb::Counters last{};   // of the launch before: its pair count sizes the next one's pair buffers
+    if (e.hCounters) last = *e.hCounters;
+    if (e.hCounters) cudaFreeHost(e.hCounters);
     e.hFrames = nullptr;
-    e.hStates = nullptr;
-    e.hBases = nullptr;
+    e.hCounters = nullptr;
     e.hCap = 0;
     const int cap = std::max(nf, 1);
-    FDZB_CUDA(cudaMallocHost(&e.hFrames, sizeof(fdzb::FrameDesc) * cap));
-    FDZB_CUDA(cudaMallocHost(&e.hStates, sizeof(fdzb::FrameState) * cap));
-    FDZB_CUDA(cudaMallocHost(&e.hBases, sizeof(int) * 3 * cap));
+    FDZB_CUDA(cudaMallocHost(&e.hFrames, frames_bytes(cap) + sizeof(int) * 3 * cap));
+    FDZB_CUDA(cudaMallocHost(&e.hCounters, kCountersBytes + sizeof(fdzb::FrameState) * cap));
+    std::memset(e.hCounters, 0, kCountersBytes + sizeof(fdzb::FrameState) * cap);
+    *e.hCounters = last;
+    e.hStates = (fdzb::FrameState *)((char *)e.hCounters + kCountersBytes);
     e.hCap = cap;
+    e.hBases = (int *)((char *)e.hFrames + frames_bytes(nf));
     return FDZB_OK;
 }
 
@@ -225,7 +235,9 @@ int engine_init(Engine &e, int device)
     FDZB_CUDA(cudaEventCreate(&e.ev0));
     FDZB_CUDA(cudaEventCreate(&e.ev1));
     for (auto &ev : e.stageEv) FDZB_CUDA(cudaEventCreate(&ev));
-    FDZB_CUDA(cudaMallocHost(&e.hCounters, sizeof(fdzb::Counters)));
+    FDZB_CUDA(cudaStreamCreateWithFlags(&e.fork.stream, cudaStreamNonBlocking));
+    for (cudaEvent_t *ev : {&e.fork.setup, &e.fork.keys, &e.fork.order, &e.fork.samples})
+        FDZB_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
     return ensure_host(e, 1);
 }
 
@@ -235,14 +247,15 @@ void engine_release(Engine &e)
     drop_graph(e);
     if (e.arena) cudaFree(e.arena);
     if (e.hFrames) cudaFreeHost(e.hFrames);
-    if (e.hStates) cudaFreeHost(e.hStates);
-    if (e.hBases) cudaFreeHost(e.hBases);
     if (e.hCounters) cudaFreeHost(e.hCounters);
     if (e.passMasks) cudaFree(e.passMasks);
     if (e.ev0) cudaEventDestroy(e.ev0);
     if (e.ev1) cudaEventDestroy(e.ev1);
     for (auto &ev : e.stageEv)
         if (ev) cudaEventDestroy(ev);
+    for (cudaEvent_t ev : {e.fork.setup, e.fork.keys, e.fork.order, e.fork.samples})
+        if (ev) cudaEventDestroy(ev);
+    if (e.fork.stream) cudaStreamDestroy(e.fork.stream);
     if (e.ownStream) cudaStreamDestroy(e.ownStream);
     e = Engine{};
 }
@@ -278,13 +291,14 @@ cudaError_t enqueue_body(Engine &e, int nf)
     fdzb::DeviceBuffers &b = e.buf;
     cudaStream_t s = e.stream;
     cudaError_t err;
-    if ((err = cudaMemcpyAsync(b.frames, e.hFrames, sizeof(fdzb::FrameDesc) * nf, cudaMemcpyHostToDevice, s))) return err;
-    if ((err = cudaMemcpyAsync(b.sampleBases, e.hBases, 3 * sizeof(int) * nf, cudaMemcpyHostToDevice, s))) return err;
-    if ((err = cudaMemsetAsync(b.counters, 0, sizeof(fdzb::Counters), s))) return err;
-    if ((err = cudaMemsetAsync(b.sortHist, 0, 4 * fdzb::kSortSlots * 256 * sizeof(uint32_t), s))) return err;
-    if ((err = fdzb::run_pipeline(b, e.maxS, e.maxT, e.maxV, s, e.profile ? e.stageEv : nullptr, &e.launches))) return err;
-    if ((err = cudaMemcpyAsync(e.hCounters, b.counters, sizeof(fdzb::Counters), cudaMemcpyDeviceToHost, s))) return err;
-    return cudaMemcpyAsync(e.hStates, b.states, sizeof(fdzb::FrameState) * nf, cudaMemcpyDeviceToHost, s);
+    if ((err = cudaMemcpyAsync(b.frames, e.hFrames, frames_bytes(nf) + 3 * sizeof(int) * nf, cudaMemcpyHostToDevice, s)))
+        return err;
+    // stage timing and debug copies want the stages one after the other
+    const bool fork = !e.profile && !e.debug;
+    if ((err = fdzb::run_pipeline(b, e.maxS, e.maxT, e.maxV, s, e.profile ? e.stageEv : nullptr, &e.launches,
+                                  fork ? &e.fork : nullptr)))
+        return err;
+    return cudaMemcpyAsync(e.hCounters, b.counters, kCountersBytes + sizeof(fdzb::FrameState) * nf, cudaMemcpyDeviceToHost, s);
 }
 
 // Clears the look-back status words and the epoch word when the arena's layout
@@ -293,12 +307,13 @@ cudaError_t enqueue_body(Engine &e, int nf)
 cudaError_t refresh_lookback(Engine &e)
 {
     const fdzb::DeviceBuffers &b = e.buf;
-    const auto where = std::make_tuple((const void *)b.sortStatus, b.sortStatusTiles, (const void *)b.triScanStatus,
-                                       b.totalTris, (const void *)b.epochWord);
+    const auto where = std::make_tuple((const void *)b.sortStatus, b.sortStatusTiles + b.auxStatusTiles,
+                                       (const void *)b.triScanStatus, b.totalTris, (const void *)b.epochWord);
     if (where != e.statusLayout || e.epochCount >= kEpochLimit) {
         const size_t triTiles = ((size_t)std::max(b.totalTris, 1) + fdzb::kTriTileHost - 1) / fdzb::kTriTileHost;
         cudaError_t err;
         if ((err = cudaMemsetAsync(b.sortStatus, 0, 8 * 256 * b.sortStatusTiles, e.stream))) return err;
+        if ((err = cudaMemsetAsync(b.auxStatus, 0, 8 * 256 * b.auxStatusTiles, e.stream))) return err;
         if ((err = cudaMemsetAsync(b.triScanStatus, 0, 8 * triTiles, e.stream))) return err;
         if ((err = cudaMemsetAsync(b.epochWord, 0, sizeof(uint32_t), e.stream))) return err;
         e.epochCount = 0;

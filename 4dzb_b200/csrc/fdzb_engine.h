@@ -81,14 +81,17 @@ struct Engine {
     std::vector<std::pair<long long, long long>> passPlan;
     std::tuple<const void *, const void *, int, int, const void *, const void *, size_t, int, int, long long>
         passKey{};
-    // pinned host staging, grown to the largest frame list
+    // pinned host staging, grown to the largest frame list: the frame table with
+    // the base offsets behind it, and the counters with the frame states behind
+    // them, each in the layout of its device block (one copy each way)
     FrameDesc *hFrames = nullptr;
-    FrameState *hStates = nullptr;
     int *hBases = nullptr;
-    int hCap = 0;
     Counters *hCounters = nullptr;
+    FrameState *hStates = nullptr;
+    int hCap = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t stageEv[STAGE_COUNT + 1] = {};
+    ForkStream fork{};      // second stream of a launch (run_pipeline)
     // the frame list of the pending / last launch
     std::vector<FrameSpec> frames;
     int maxS = 0, maxT = 0, maxV = 0;

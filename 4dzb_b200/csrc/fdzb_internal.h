@@ -83,7 +83,8 @@ struct FrameState {
     float fx, fy;
     float sampleAabb[6], modelAabb[6];
     int quirkKeyRange;
-    int pad[3];
+    int arrived;            // blocks of k_reduce that are done (the last one plans the frame)
+    int pad[2];
 };
 
 // Launch-wide counters and error word (zeroed every launch).
@@ -140,8 +141,10 @@ struct DeviceBuffers {
     uint32_t *tkeysA, *tvalsA, *tkeysB, *tvalsB;  // [totalTris]
     // sort scratch
     uint32_t *sortHist;                         // [12 * 256]: 4 sample, 4 pair, 4 triangle passes
-    unsigned long long *sortStatus;             // [sortStatusTiles * 256] epoch-tagged
-    size_t sortStatusTiles;
+    // look-back words, epoch-tagged: [sortStatusTiles * 256] of the pair sort and
+    // [auxStatusTiles * 256] of the sample and triangle sorts, which run beside it
+    unsigned long long *sortStatus, *auxStatus;
+    size_t sortStatusTiles, auxStatusTiles;
     int *sampleBases, *triBases, *binBases;     // [nframes] ascending global bases
     // occlusion work list
     int4 *items;                                // [itemCapacity]
@@ -174,8 +177,14 @@ void light_setup(const float rightRadius, const float topRadius, const float pos
 // maxS / maxT / maxV: largest per-frame sample / triangle / vertex counts.
 // stageEvents: nullptr, or STAGE_COUNT + 1 events recorded at the stage
 // boundaries.  *launches receives the number of kernels enqueued.
+// fork: nullptr, or a second stream and the events that tie it to `stream`, on
+// which the triangle and sample sorts run beside the pair stages.
+struct ForkStream {
+    cudaStream_t stream;
+    cudaEvent_t setup, keys, order, samples;   // ends of k_tri_setup, k_sample_keys, the two sorts
+};
 cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, cudaStream_t stream,
-                         cudaEvent_t *stageEvents, int *launches);
+                         cudaEvent_t *stageEvents, int *launches, const ForkStream *fork);
 // Issue-rate probe: lane FP32 adds per second of a kernel with independent chains.
 cudaError_t measure_alu_rate(double *laneOpsPerSecond);
 cudaError_t check_division(unsigned long long trials, unsigned long long seed, unsigned long long *mismatches,

@@ -1,14 +1,14 @@
 // fdzb_pipeline.cu -- the B200 FDZB soft-shadow pipeline.
 //
 // Stage map (reference kernels in 4DZB/FDZB_Soft_Shadow/cuda/, "K/"):
-//   k_init        clears per-launch bin state
+//   k_init        clears per-launch bin state, counters and digit histograms
 //   k_reduce      k1+k2+k3+k4 fused: one pass over samples (pos+normal, 128-bit
 //                 loads) and vertices computes the far-plane depth maxima and the
-//                 sample / vertex rectangle bounds (K/Step2_1_*, K/Step2_2_*)
-//   k_plan        light plane, far plane f, sub-constant, bin factor
-//                 (K/Step2_3_defineFDbuffer.inl:5-111)
+//                 sample / vertex rectangle bounds (K/Step2_1_*, K/Step2_2_*); the
+//                 frame's last block plans it: light plane, far plane f,
+//                 sub-constant, bin factor (K/Step2_3_defineFDbuffer.inl:5-111)
 //   k_tri_setup   per-triangle cull + footprint AABB + 64-byte record
-//                 (K/Step0_triangleSetup.inl:37-191)
+//                 (K/Step0_triangleSetup.inl:37-191) and coverage-order key
 //   k_sample_keys bin key per sample, back-facing/unbinned outputs, per-bin
 //                 sample stats by warp-aggregated atomics (k6 + k9,
 //                 K/Step3_bindSampleToBin.inl:5-104)
@@ -45,11 +45,16 @@ __device__ __forceinline__ f3 load_vertex(const FrameDesc &fr, int v)
 // segment tables (K/binRaster.inl:39-40, 52-53).
 // ---------------------------------------------------------------------------
 __global__ void k_init(FrameState *states, int nframes, uint32_t *binStat, int32_t *bss,
-                       int32_t *bse, int32_t *bts, int32_t *bte, int totalBins, uint32_t *epochWord)
+                       int32_t *bse, int32_t *bts, int32_t *bte, int totalBins, uint32_t *epochWord,
+                       Counters *counters, uint32_t *sortHist)
 {
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid == 0) *epochWord += 1u;  // launch number: look-back tags of this launch
     const int stride = gridDim.x * blockDim.x;
+    static_assert(sizeof(Counters) % sizeof(uint32_t) == 0, "counters cleared word by word");
+    for (int i = gid; i < (int)(sizeof(Counters) / sizeof(uint32_t)); i += stride)
+        reinterpret_cast<uint32_t *>(counters)[i] = 0u;
+    for (int i = gid; i < 4 * kSortSlots * kRadix; i += stride) sortHist[i] = 0u;
     const uint32_t neg = f2o(-kF32Max), pos = f2o(kF32Max);
     for (int b = gid; b < totalBins; b += stride) {
         uint4 s0 = make_uint4(neg, neg, neg, pos);
@@ -76,7 +81,60 @@ __global__ void k_init(FrameState *states, int nframes, uint32_t *binStat, int32
         s.nValidTris = 0;
         s.nValidSamples = 0;
         s.quirkKeyRange = 0;
+        s.arrived = 0;
     }
+}
+
+// ---------------------------------------------------------------------------
+// The frame's plan: host logic of lightPlaneParamCal
+// (K/Step2_3_defineFDbuffer.inl:14-104) with the early exits as frame states.
+// Run by one thread of the frame's last k_reduce block, after every block's
+// atomics; the bounds are read past the L1 cache for that reason.
+// ---------------------------------------------------------------------------
+__device__ void plan_frame(const FrameDesc &fr, FrameState &st)
+{
+    uint32_t acc[ACC_COUNT];
+    for (int i = 0; i < ACC_COUNT; ++i) acc[i] = __ldcg(&st.acc[i]);
+    const int nFront = __ldcg(&st.nFront);
+    const float smax = o2f(acc[ACC_SMAXW]);
+    const float tmax = o2f(acc[ACC_TMAXW]);
+    st.state = 0;
+    if (smax < 0.0f || tmax < 0.0f) return;
+    const float f = __fadd_rn(fmaxf(smax, tmax), 0.1f);
+    const float subx = __fdiv_rn(fr.light.RF[0], f), suby = __fdiv_rn(fr.light.RF[1], f);
+    st.f = f;
+    st.subx = subx;
+    st.suby = suby;
+    st.state = 1;
+    float s[6], m[6];
+    s[0] = o2f(acc[ACC_S_MINU]);
+    s[1] = o2f(acc[ACC_S_MINV]);
+    s[2] = o2f(acc[ACC_S_MINW]);
+    s[3] = nFront ? __fsub_rn(o2f(acc[ACC_S_MAXA]), subx) : -kF32Max;
+    s[4] = nFront ? __fsub_rn(o2f(acc[ACC_S_MAXB]), suby) : -kF32Max;
+    s[5] = o2f(acc[ACC_S_MAXW]);
+    m[0] = o2f(acc[ACC_M_MINU]);
+    m[1] = o2f(acc[ACC_M_MINV]);
+    m[2] = o2f(acc[ACC_M_MINW]);
+    m[3] = fr.V ? __fsub_rn(o2f(acc[ACC_M_MAXA]), subx) : -kF32Max;
+    m[4] = fr.V ? __fsub_rn(o2f(acc[ACC_M_MAXB]), suby) : -kF32Max;
+    m[5] = o2f(acc[ACC_M_MAXW]);
+    for (int i = 0; i < 6; ++i) {
+        st.sampleAabb[i] = s[i];
+        st.modelAabb[i] = m[i];
+    }
+    if (nFront == 0) return;  // K/Step2_1_samplerRectangleAABB.inl:178-181
+    if (m[0] > m[3] || m[1] > m[4] || s[0] > s[3] || s[1] > s[4]) return;
+    st.Bx = fmaxf(s[0], m[0]);
+    st.By = fmaxf(s[1], m[1]);
+    st.Ex = fminf(s[3], m[3]);
+    st.Ey = fminf(s[4], m[4]);
+    st.Bz = m[2];
+    st.Ez = s[5];
+    if (st.Bx >= st.Ex || st.By >= st.Ey) return;
+    st.fx = __fdiv_rn((float)fr.Wb, __fsub_rn(st.Ex, st.Bx));
+    st.fy = __fdiv_rn((float)fr.Wb, __fsub_rn(st.Ey, st.By));
+    st.state = 2;
 }
 
 // ---------------------------------------------------------------------------
@@ -85,7 +143,8 @@ __global__ void k_init(FrameState *states, int nframes, uint32_t *binStat, int32
 // front-facing samples.  The bound on rect.x + RF.x/w - sub is reduced before
 // the subtraction (sub = RF/f needs f first): fl(x - sub) is monotone in x, so
 // max_i fl(a_i - sub) == fl(max_i a_i - sub) exactly.
-// Vertex part: k2 (max depth) and k4 (vertex rectangle bounds).
+// Vertex part: k2 (max depth) and k4 (vertex rectangle bounds).  The frame's
+// last block plans it (a launch of its own before: 3 us and a gap).
 // ---------------------------------------------------------------------------
 constexpr int kReduceThreads = 256;
 
@@ -184,67 +243,53 @@ __global__ void __launch_bounds__(kReduceThreads)
             for (int k = 0; k < kReduceThreads / 32; ++k) t += s_cnt[k];
             if (t) atomicAdd(&st.nFront, t);
         }
+        __threadfence();
     }
-}
-
-// ---------------------------------------------------------------------------
-// k_plan: one thread per frame; host logic of lightPlaneParamCal
-// (K/Step2_3_defineFDbuffer.inl:14-104) with the early exits as frame states.
-// ---------------------------------------------------------------------------
-__global__ void k_plan(const FrameDesc *__restrict__ frames, FrameState *states, int nframes)
-{
-    const int fi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (fi >= nframes) return;
-    const FrameDesc &fr = frames[fi];
-    FrameState &st = states[fi];
-    const float smax = o2f(st.acc[ACC_SMAXW]);
-    const float tmax = o2f(st.acc[ACC_TMAXW]);
-    st.state = 0;
-    if (smax < 0.0f || tmax < 0.0f) return;
-    const float f = __fadd_rn(fmaxf(smax, tmax), 0.1f);
-    const float subx = __fdiv_rn(fr.light.RF[0], f), suby = __fdiv_rn(fr.light.RF[1], f);
-    st.f = f;
-    st.subx = subx;
-    st.suby = suby;
-    st.state = 1;
-    float s[6], m[6];
-    s[0] = o2f(st.acc[ACC_S_MINU]);
-    s[1] = o2f(st.acc[ACC_S_MINV]);
-    s[2] = o2f(st.acc[ACC_S_MINW]);
-    s[3] = st.nFront ? __fsub_rn(o2f(st.acc[ACC_S_MAXA]), subx) : -kF32Max;
-    s[4] = st.nFront ? __fsub_rn(o2f(st.acc[ACC_S_MAXB]), suby) : -kF32Max;
-    s[5] = o2f(st.acc[ACC_S_MAXW]);
-    m[0] = o2f(st.acc[ACC_M_MINU]);
-    m[1] = o2f(st.acc[ACC_M_MINV]);
-    m[2] = o2f(st.acc[ACC_M_MINW]);
-    m[3] = fr.V ? __fsub_rn(o2f(st.acc[ACC_M_MAXA]), subx) : -kF32Max;
-    m[4] = fr.V ? __fsub_rn(o2f(st.acc[ACC_M_MAXB]), suby) : -kF32Max;
-    m[5] = o2f(st.acc[ACC_M_MAXW]);
-    for (int i = 0; i < 6; ++i) {
-        st.sampleAabb[i] = s[i];
-        st.modelAabb[i] = m[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int blocks = (int)(gridDim.x * gridDim.z);
+        if (atomicAdd(&st.arrived, 1) == blocks - 1) {
+            __threadfence();
+            plan_frame(fr, st);
+        }
     }
-    if (st.nFront == 0) return;  // K/Step2_1_samplerRectangleAABB.inl:178-181
-    if (m[0] > m[3] || m[1] > m[4] || s[0] > s[3] || s[1] > s[4]) return;
-    st.Bx = fmaxf(s[0], m[0]);
-    st.By = fmaxf(s[1], m[1]);
-    st.Ex = fminf(s[3], m[3]);
-    st.Ey = fminf(s[4], m[4]);
-    st.Bz = m[2];
-    st.Ez = s[5];
-    if (st.Bx >= st.Ex || st.By >= st.Ey) return;
-    st.fx = __fdiv_rn((float)fr.Wb, __fsub_rn(st.Ex, st.Bx));
-    st.fy = __fdiv_rn((float)fr.Wb, __fsub_rn(st.Ey, st.By));
-    st.state = 2;
 }
 
 // ---------------------------------------------------------------------------
 // k_tri_setup: grid (x, frame).  Record layout (4 x float4 = 64 B):
 //   q0 = (v0, minz) q1 = (v1, maxz) q2 = (v2, 0) q3 = (aabb min x,y, aabb max x,y)
-// and the edge-mask kernel's record (FastTri, 4 x float4).
+// and the edge-mask kernel's record (FastTri, 4 x float4); with depthBits > 0 the
+// coverage order's sort input too, (bucket, triangle id), and its digit counts
+// (a launch each of their own before).
 // Culled triangles keep the inverted AABB of the reference's triAABB buffer, so
 // the pair counter's skip test rejects them exactly as K/Step4_*.inl:41 does.
 // ---------------------------------------------------------------------------
+// Coverage-order bucket of a triangle (the key of the triangle sort): the triangle's
+// angular size seen from below, world area / (f - minz)^2 with f - minz the
+// light-depth distance from the far plane (about the receivers' depth) to the
+// triangle's vertex nearest the light, as a log-scale bucket; the largest
+// come first.  A sample's mask is the OR over its bin's triangles, so the order
+// changes only how soon its light rows fill (the early-out), never the result.
+__device__ __forceinline__ uint32_t coverage_bucket(f3 v0, f3 v1, f3 v2, float minz, float f, int depthBits)
+{
+    const float ax = v1.x - v0.x, ay = v1.y - v0.y, az = v1.z - v0.z;
+    const float bx = v2.x - v0.x, by = v2.y - v0.y, bz = v2.z - v0.z;
+    const float cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
+    const float area2 = fmaxf(sqrtf(cx * cx + cy * cy + cz * cz), 1e-30f);
+    const float d = fmaxf(f - minz, 1e-6f);   // minz: the triangle's least light depth
+    const float nb = (float)(1 << depthBits);
+    const float q = -log2f(area2 / (d * d)) * (nb / 40.0f) + 0.5f * nb;
+    return (uint32_t)(int)fminf(fmaxf(q, 0.0f), nb - 1.0f);
+}
+
+// Adds a block's digit counts of a sort's keys to the sort's histogram.
+__device__ __forceinline__ void flush_hist(const uint32_t *s_hist, int n, uint32_t *__restrict__ hist)
+{
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+}
+
 // The fast record of a triangle that was not culled (FastTri).
 __device__ __forceinline__ void store_fast_tri(float4 *__restrict__ o, const LightParams &L, f3 v0, f3 v1, f3 v2,
                                                float4 aabb, float minz, float maxz)
@@ -271,11 +316,27 @@ __device__ __forceinline__ void store_fast_tri(float4 *__restrict__ o, const Lig
 
 __global__ void __launch_bounds__(256)
     k_tri_setup(const FrameDesc *__restrict__ frames, FrameState *states, float4 *__restrict__ rec,
-                float4 *__restrict__ fast, int *err)
+                float4 *__restrict__ fast, int *err, int depthBits, int passes, uint32_t *__restrict__ orderKeys,
+                uint32_t *__restrict__ orderVals, uint32_t *__restrict__ orderHist)
 {
+    __shared__ uint32_t s_hist[2 * kRadix];
     const FrameDesc &fr = frames[blockIdx.y];
     FrameState &st = states[blockIdx.y];
-    if (st.state < 2) return;
+    for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) s_hist[i] = 0;
+    __syncthreads();
+    // a triangle's place in the coverage order: its bucket, counted for the sort
+    auto order = [&](int t, uint32_t key) {
+        if (depthBits <= 0) return;
+        orderKeys[fr.triBase + t] = key;
+        orderVals[fr.triBase + t] = (uint32_t)(fr.triBase + t);
+        for (int p = 0; p < passes; ++p) atomicAdd(&s_hist[p * kRadix + ((key >> (8 * p)) & 255u)], 1u);
+    };
+    if (st.state < 2) {   // no light plane: the frame emits no pairs, its triangles go last
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < fr.T; t += gridDim.x * blockDim.x)
+            order(t, (1u << depthBits) - 1u);
+        if (depthBits > 0) flush_hist(s_hist, passes * kRadix, orderHist);
+        return;
+    }
     const float *M = fr.light.mat;
     const float RFx = fr.light.RF[0], RFy = fr.light.RF[1];
     const float subx = st.subx, suby = st.suby;
@@ -328,24 +389,35 @@ __global__ void __launch_bounds__(256)
             o[1] = make_float4(v1.x, v1.y, v1.z, mxz);
             o[2] = make_float4(v2.x, v2.y, v2.z, 0.0f);
             o[3] = make_float4(mnx, mny, mxx, mxy);
+            order(t, depthBits > 0 ? coverage_bucket(v0, v1, v2, mnz, st.f, depthBits) : 0u);
             if (mnx <= mxx) store_fast_tri(fast + 4 * (size_t)(fr.triBase + t), fr.light, v0, v1, v2, o[3], mnz, mxz);
         }
         const unsigned b = __ballot_sync(kFullWarp, inLP);
         if (lane == 0 && b) atomicAdd(&st.nValidTris, __popc(b));
     }
+    if (depthBits > 0) flush_hist(s_hist, passes * kRadix, orderHist);
 }
 
 // ---------------------------------------------------------------------------
 // k_sample_keys: grid (x, frame).  k3's back-face/validity decision and
 // rectangle, k6's key (K/Step3_bindSampleToBin.inl:29-57) and k9's per-bin
 // statistics (max w, max rect.min x/y, min rect.max x/y; :61-104) by
-// warp-aggregated atomics on order-preserving encodings.  Samples that get no
+// warp-aggregated atomics on order-preserving encodings, and the digit counts of
+// the sample sort, one per distinct key and warp as well.  Samples that get no
 // bin receive their final output here: 1 (full mask) if back-facing, else 0.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     k_sample_keys(const FrameDesc *__restrict__ frames, FrameState *states, uint32_t *__restrict__ keys,
-                  uint32_t *__restrict__ vals, uint32_t *binStat, int invalidKey)
+                  uint32_t *__restrict__ vals, uint32_t *binStat, int invalidKey, int passes,
+                  uint32_t *__restrict__ keyHist)
 {
+    __shared__ uint32_t s_hist[4 * kRadix];
+    for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) s_hist[i] = 0;
+    __syncthreads();
+    // n samples of a key, counted for the sort's passes
+    auto count = [&](uint32_t key, int n) {
+        for (int p = 0; p < passes; ++p) atomicAdd(&s_hist[p * kRadix + ((key >> (8 * p)) & 255u)], (uint32_t)n);
+    };
     const FrameDesc &fr = frames[blockIdx.y];
     FrameState &st = states[blockIdx.y];
     const int state = st.state;
@@ -419,6 +491,8 @@ __global__ void __launch_bounds__(256)
         }
         // per-bin statistics, one atomic per distinct key per warp
         unsigned todo = __ballot_sync(kFullWarp, valid);
+        const unsigned none = __ballot_sync(kFullWarp, in && !valid);
+        if (lane == 0 && none) count((uint32_t)invalidKey, __popc(none));
         nvalid += valid ? 1 : 0;
         while (todo) {
             const int leader = __ffs(todo) - 1;
@@ -437,6 +511,7 @@ __global__ void __launch_bounds__(256)
                 atomicMax(s + 2, ry);
                 atomicMin(s + 3, rz);
                 atomicMin(s + 4, rw);
+                count(lk, __popc(grp));
             }
             todo &= ~grp;
         }
@@ -447,6 +522,7 @@ __global__ void __launch_bounds__(256)
         if (nvalid) atomicAdd(&st.nValidSamples, nvalid);
         if (nquirk) atomicAdd(&st.quirkKeyRange, nquirk);
     }
+    flush_hist(s_hist, passes * kRadix, keyHist);
 }
 
 // ---------------------------------------------------------------------------
@@ -506,42 +582,6 @@ __device__ __forceinline__ bool stat_accepts(uint4 s, uint32_t s4, const TriBins
 {
     const float maxz = o2f(s.x), Rx = o2f(s.y), Ry = o2f(s.z), Rz = o2f(s.w), Rw = o2f(s4);
     return maxz >= c.bz && c.bx < Rx && c.by < Ry && Rz < c.ex && Rw < c.ey;
-}
-
-// Coverage-order bucket of a triangle (the key of the triangle sort): the triangle's
-// angular size seen from below, world area / (f - minz)^2 with f - minz the
-// light-depth distance from the far plane (about the receivers' depth) to the
-// triangle's vertex nearest the light, as a log-scale bucket; the largest
-// come first.  A sample's mask is the OR over its bin's triangles, so the order
-// changes only how soon its light rows fill (the early-out), never the result.
-__device__ __forceinline__ uint32_t coverage_bucket(const float4 *__restrict__ rec, int g, float f, int depthBits)
-{
-    if (depthBits <= 0) return 0u;   // reference order: the reference's (bin, triangle) order
-    const float4 r0 = __ldg(&rec[4 * (size_t)g]), r1 = __ldg(&rec[4 * (size_t)g + 1]),
-                 r2 = __ldg(&rec[4 * (size_t)g + 2]);
-    const float ax = r1.x - r0.x, ay = r1.y - r0.y, az = r1.z - r0.z;
-    const float bx = r2.x - r0.x, by = r2.y - r0.y, bz = r2.z - r0.z;
-    const float cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
-    const float area2 = fmaxf(sqrtf(cx * cx + cy * cy + cz * cz), 1e-30f);
-    const float d = fmaxf(f - r0.w, 1e-6f);   // r0.w: the triangle's least light depth
-    const float nb = (float)(1 << depthBits);
-    const float q = -log2f(area2 / (d * d)) * (nb / 40.0f) + 0.5f * nb;
-    return (uint32_t)(int)fminf(fmaxf(q, 0.0f), nb - 1.0f);
-}
-
-// k_tri_order: the coverage order's sort input, (bucket, triangle id) for every
-// triangle; triangles of frames without a light plane go last (they emit no
-// pairs either way).
-__global__ void k_tri_order(const FrameState *__restrict__ states, const int *__restrict__ triBases, int nframes,
-                            int totalTris, const float4 *__restrict__ rec, int depthBits,
-                            uint32_t *__restrict__ keys, uint32_t *__restrict__ vals)
-{
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < totalTris; g += gridDim.x * blockDim.x) {
-        const FrameState &st = states[frame_of(triBases, nframes, g)];
-        keys[g] = (st.state == 2 && st.nValidTris > 0) ? coverage_bucket(rec, g, st.f, depthBits)
-                                                       : (1u << depthBits) - 1u;
-        vals[g] = (uint32_t)g;
-    }
 }
 
 // Candidate bins of a triangle, swept by a warp 32 at a time in row-major
@@ -843,13 +883,16 @@ static_assert(kKeysTile >= kSortTile, "the look-back status array is sized for t
 // 16*launch + 4*slot + p and the key's bits [shift0 + 8p, shift0 + 8p + 8).
 // vA == nullptr: keys alone.  With segStart/segEnd the last pass also writes
 // the bounds of the segments key >> segShift (nslots of them; K/binRaster.inl:5-33).
+// The digit counts are in the slot's histogram already where the keys' producer
+// made them (slots 0 and 2); the pair sort's are counted here.
 static void run_sort(const DeviceBuffers &b, int slot, uint32_t *kA, uint32_t *vA, uint32_t *kB,
                      uint32_t *vB, const int *n_dev, int n_static, int cap, int passes, int sm,
                      cudaStream_t s, int shift0 = 0, int32_t *segStart = nullptr, int32_t *segEnd = nullptr,
                      int segShift = 0, uint32_t nslots = 0)
 {
     uint32_t *hist = b.sortHist + slot * 4 * kRadix;
-    k_radix_hist<<<grid_for(cap, kSortThreads, sm * 4), kSortThreads, 0, s>>>(kA, n_dev, n_static,
+    unsigned long long *status = slot == 1 ? b.sortStatus : b.auxStatus;
+    if (slot == 1) k_radix_hist<<<grid_for(cap, kSortThreads, sm * 4), kSortThreads, 0, s>>>(kA, n_dev, n_static,
                                                                               cap, passes, shift0, hist);
     uint32_t *ki = kA, *vi = vA, *ko = kB, *vo = vB;
     const long long tiles = ((long long)cap + kSortTile - 1) / kSortTile;
@@ -859,7 +902,7 @@ static void run_sort(const DeviceBuffers &b, int slot, uint32_t *kA, uint32_t *v
     for (int p = 0; p < passes; ++p) {
         const bool seg = segStart && p == passes - 1;
 #define FDZB_PASS_ARGS(VI, VO)                                                                               \
-    ki, VI, ko, VO, n_dev, n_static, cap, shift0 + 8 * p, hist + p * kRadix, b.sortStatus, b.epochWord,      \
+    ki, VI, ko, VO, n_dev, n_static, cap, shift0 + 8 * p, hist + p * kRadix, status, b.epochWord,      \
         (uint32_t)(slot * 4 + p), b.counters->sortTileCounter + slot * 4 + p, &b.counters->errorFlags
         if (vA && seg)
             k_radix_pass<true, kSortItems, FDZB_SORT_MINBLOCKS, true><<<passGrid, kSortThreads, 0, s>>>(
@@ -897,7 +940,7 @@ static int sm_count()
 }
 
 cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, cudaStream_t s,
-                         cudaEvent_t *ev, int *launches)
+                         cudaEvent_t *ev, int *launches, const ForkStream *fork)
 {
     const int sm = sm_count();
     const int nf = b.nframes;
@@ -906,37 +949,60 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     // (a) samples, vertices, triangles
     k_init<<<grid_for(b.totalBins + 1, 256, sm * 8), 256, 0, s>>>(
         b.states, nf, b.binStat, b.binSampleStart, b.binSampleEnd, b.binTriStart, b.binTriEnd, b.totalBins,
-        b.epochWord);
+        b.epochWord, b.counters, b.sortHist);
     {
         const int gx = grid_for(maxS > maxV ? maxS : maxV, kReduceThreads, sm * 4);
         k_reduce<<<dim3(gx, nf, 2), kReduceThreads, 0, s>>>(b.frames, b.states);
     }
-    k_plan<<<(nf + 63) / 64, 64, 0, s>>>(b.frames, b.states, nf);
-    k_tri_setup<<<dim3(grid_for(maxT, 256, sm * 8), nf), 256, 0, s>>>(b.frames, b.states, b.triRec,
-                                                                      b.triFast, &b.counters->errorFlags);
+    const bool ordered = b.depthBits > 0 && b.totalTris > 0;
+    k_tri_setup<<<dim3(grid_for(maxT, 256, sm * 8), nf), 256, 0, s>>>(
+        b.frames, b.states, b.triRec, b.triFast, &b.counters->errorFlags, ordered ? b.depthBits : 0, b.triPasses,
+        b.tkeysA, b.tvalsA, b.sortHist + 2 * 4 * kRadix);
+    // The sorts of triangles and samples run beside what does not need them: the
+    // triangles' beside the sample keys, the samples' beside the pair stages (the
+    // occlusion stage is the first to read it).  Small frames are a chain of short
+    // launches (128 x 96 samples: 57 of 146 us in these two sorts); large ones lose
+    // nothing.  Without a second stream: one after the other.
+    cudaStream_t s2 = fork ? fork->stream : s;
+    auto sample_sort = [&]() {
+        run_sort(b, 0, b.keysA, b.valsA, b.keysB, b.valsB, nullptr, b.totalSamples, b.totalSamples,
+                 b.samplePasses, sm, s2, 0, b.binSampleStart, b.binSampleEnd, 0, (uint32_t)b.totalBins + 1u);
+    };
+    auto triangle_sort = [&]() {
+        run_sort(b, 2, b.tkeysA, b.tvalsA, b.tkeysB, b.tvalsB, nullptr, b.totalTris, b.totalTris, b.triPasses, sm, s2);
+    };
+    if (fork) {
+        cudaEventRecord(fork->setup, s);
+        cudaStreamWaitEvent(s2, fork->setup, 0);
+        if (ordered) triangle_sort();
+        cudaEventRecord(fork->order, s2);
+    }
     k_sample_keys<<<dim3(grid_for(maxS, 256, sm * 8), nf), 256, 0, s>>>(
-        b.frames, b.states, b.keysA, b.valsA, b.binStat, b.totalBins);
-    nl += 5;
+        b.frames, b.states, b.keysA, b.valsA, b.binStat, b.totalBins, b.samplePasses, b.sortHist);
     if (b.dbgKeys) {
         cudaMemcpyAsync(b.dbgKeys, b.keysA, 4ull * b.totalSamples, cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(b.dbgVals, b.valsA, 4ull * b.totalSamples, cudaMemcpyDeviceToDevice, s);
     }
     // (b) sample sort and segments
     if (ev) cudaEventRecord(ev[STAGE_SAMPLE_SORT], s);
-    run_sort(b, 0, b.keysA, b.valsA, b.keysB, b.valsB, nullptr, b.totalSamples, b.totalSamples,
-             b.samplePasses, sm, s, 0, b.binSampleStart, b.binSampleEnd, 0, (uint32_t)b.totalBins + 1u);
+    if (fork) {
+        cudaEventRecord(fork->keys, s);
+        cudaStreamWaitEvent(s2, fork->keys, 0);
+        sample_sort();
+        cudaEventRecord(fork->samples, s2);
+        cudaStreamWaitEvent(s, fork->order, 0);
+    } else {
+        sample_sort();
+    }
     uint32_t *sv = (b.samplePasses & 1) ? b.valsB : b.valsA;
-    nl += 1 + b.samplePasses;
+    nl += 4 + b.samplePasses;
     // (a) triangle/bin pairs, in the coverage order when one is asked for
     if (ev) cudaEventRecord(ev[STAGE_TRI_PAIRS], s);
     const uint32_t *order = nullptr;
-    if (b.depthBits > 0 && b.totalTris > 0) {
-        k_tri_order<<<grid_for(b.totalTris, 256, sm * 8), 256, 0, s>>>(b.states, b.triBases, nf, b.totalTris,
-                                                                     b.triRec, b.depthBits, b.tkeysA, b.tvalsA);
-        run_sort(b, 2, b.tkeysA, b.tvalsA, b.tkeysB, b.tvalsB, nullptr, b.totalTris, b.totalTris, b.triPasses,
-                 sm, s);
+    if (ordered) {
+        if (!fork) triangle_sort();
         order = (b.triPasses & 1) ? b.tvalsB : b.tvalsA;
-        nl += 2 + b.triPasses;
+        nl += b.triPasses;
     }
     {
         // tiles of 64 triangles, 8 a warp, up to a million triangles: a frame
@@ -980,6 +1046,7 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     nl += 1 + b.pairPasses;
     // (c) + (d) occlusion and shading
     if (ev) cudaEventRecord(ev[STAGE_OCCLUSION], s);
+    if (fork) cudaStreamWaitEvent(s, fork->samples, 0);
     k_items<<<grid_for(b.totalBins, 256, sm * 8), 256, 0, s>>>(
         b.frames, b.binSampleStart, b.binSampleEnd, b.binTriStart, b.binTriEnd, b.binBases, nf, b.totalBins,
         b.items, b.itemCapacity, b.counters);

@@ -3,8 +3,10 @@
 // Replaces the reference's thrust::sort_by_key calls
 // (K/Step3_bindSampleToBin.inl:125-127, K/Step4_RasterizeTriangleToBin.inl:221-223):
 // same result (keys ascending, equal keys in input order), one-sweep design:
-//   1. one histogram pass counts the 8-bit digits of every pass at once
-//      (shared-memory digit histograms, one global atomic per digit per block);
+//   1. one histogram counts the 8-bit digits of every pass at once (shared-memory
+//      digit histograms, one global atomic per digit per block): made by the kernel
+//      that writes the keys, or a pass of its own where their number is not known
+//      before (the pairs);
 //   2. one scatter pass per digit: each CTA takes the next tile ticket, ranks its
 //      keys with warp match/popc against per-warp shared histograms, publishes its
 //      per-digit tile count, and finds its global offsets by a decoupled look-back
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
                 }
             }
         }
+        if ((long long)gridDim.x * TILE >= n) break;   // a tile a block: no second ticket
     }
 }
 
