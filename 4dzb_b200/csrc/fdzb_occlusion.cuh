@@ -434,7 +434,9 @@ struct OccItem {
 
 // Takes the next item with triangles from the work queue (lane 0's ticket);
 // items of bins without triangles get their zero shadows here.  False at the
-// queue's end.
+// queue's end.  TEAM: the block's warps take one item together (thread 0's
+// ticket; every warp enters and leaves with the others).
+template <int TEAM = 0>
 __device__ __forceinline__ bool next_item(OccItem &w, const FrameDesc *__restrict__ frames,
                                           const int4 *__restrict__ items, int itemCapacity, Counters *ctr,
                                           const int32_t *__restrict__ bss, const int32_t *__restrict__ bse,
@@ -445,8 +447,16 @@ __device__ __forceinline__ bool next_item(OccItem &w, const FrameDesc *__restric
     const int nitems = min(*(volatile const int *)&ctr->itemCount, itemCapacity);
     for (;;) {
         int it = 0;
-        if (lane == 0) it = atomicAdd(&ctr->itemCursor, 1);
-        it = __shfl_sync(kFullWarp, it, 0);
+        if constexpr (TEAM) {
+            __shared__ int s_item;
+            __syncthreads();
+            if (threadIdx.x == 0) s_item = atomicAdd(&ctr->itemCursor, 1);
+            __syncthreads();
+            it = s_item;
+        } else {
+            if (lane == 0) it = atomicAdd(&ctr->itemCursor, 1);
+            it = __shfl_sync(kFullWarp, it, 0);
+        }
         if (it >= nitems) return false;
         const int4 item = items[it];
         const int bin = item.x;
@@ -463,7 +473,7 @@ __device__ __forceinline__ bool next_item(OccItem &w, const FrameDesc *__restric
         if (w.nT > 0) return true;
         // no triangle in this bin: shadow 0 -- or, in a later triangle pass,
         // the result of the earlier passes, left as it is
-        if (!fr.accumulate) {
+        if (!fr.accumulate && (!TEAM || threadIdx.x < 32)) {
             for (int k = w.sLo + lane; k < w.sHi; k += 32) {
                 const int local = (int)sortedVals[k] - fr.sampleBase;
                 if ((unsigned)local < (unsigned)(fr.W * fr.H)) write_zero(fr, local);

@@ -1068,9 +1068,17 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
         else                                                                                                 \
             k_occlusion<RT, DP, BX, 0, ROWS><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
     } while (0)
+    // team: an item for each block at the most (an item is 32 samples or more of
+    // one bin).  The counting forms and those without the cull keep a warp per item.
+    const long long mostItems = b.totalSamples / 32 + (b.totalBins < b.totalSamples ? b.totalBins : b.totalSamples);
+    const bool team = b.openBox && !b.countWork && mostItems <= (b.wide ? g64 : g32);
 #define FDZB_OCC_FORMS(RT, ROWS, G, T)                                                                        \
     do {                                                                                                     \
-        if (b.depthPlane && b.openBox) FDZB_OCC(RT, 1, 1, ROWS, G, T);                                        \
+        if (team && b.depthPlane)                                                                            \
+            k_occlusion<RT, 1, 1, 0, ROWS, 1><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
+        else if (team)                                                                                       \
+            k_occlusion<RT, 0, 1, 0, ROWS, 1><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
+        else if (b.depthPlane && b.openBox) FDZB_OCC(RT, 1, 1, ROWS, G, T);                                        \
         else if (b.depthPlane) FDZB_OCC(RT, 1, 0, ROWS, G, T);                                                \
         else if (b.openBox) FDZB_OCC(RT, 0, 1, ROWS, G, T);                                                   \
         else FDZB_OCC(RT, 0, 0, ROWS, G, T);                                                                  \
