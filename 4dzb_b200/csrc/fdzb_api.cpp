@@ -96,7 +96,8 @@ size_t layout(fdzb::DeviceBuffers &b, char *base, int nf, long long S, long long
     b.totalTris = (int)T;
     b.totalBins = (int)NB;
     b.pairCapacity = (int)P;
-    // two blocks that the host copies whole: frames and bases, counters and states
+    // one run of blocks, in the layout of the host's (HostBlock): frames, bases,
+    // counters and states go up in one copy, the last two come back in one
     b.frames = (fdzb::FrameDesc *)take(sizeof(fdzb::FrameDesc) * nf);
     b.sampleBases = (int *)take(sizeof(int) * 3 * nf);
     b.counters = (fdzb::Counters *)take(sizeof(fdzb::Counters));
@@ -116,7 +117,8 @@ size_t layout(fdzb::DeviceBuffers &b, char *base, int nf, long long S, long long
     b.triRec = (float4 *)take(64 * Ts);
     b.triFast = (float4 *)take(64 * Ts);
     b.triCount = (int32_t *)take(4 * Ts);
-    b.triScanStatus = (unsigned long long *)take(8 * ((Ts + fdzb::kTriTileHost - 1) / fdzb::kTriTileHost));
+    b.triScanTiles = (Ts + fdzb::kTriTileHost - 1) / fdzb::kTriTileHost;
+    b.triScanStatus = (unsigned long long *)take(8 * b.triScanTiles);
     b.tkeysA = (uint32_t *)take(4 * Ts);
     b.tvalsA = (uint32_t *)take(4 * Ts);
     b.tkeysB = (uint32_t *)take(4 * Ts);
@@ -127,9 +129,9 @@ size_t layout(fdzb::DeviceBuffers &b, char *base, int nf, long long S, long long
     b.pvalsB = (uint32_t *)take(4 * Ps);
     b.binTriStart = (int32_t *)take(4 * (size_t)NB);
     b.binTriEnd = (int32_t *)take(4 * (size_t)NB);
-    b.sortStatusTiles = (Ps + fdzb::kSortTileHost - 1) / fdzb::kSortTileHost;
+    b.sortStatusTiles = fdzb::sort_tiles(Ps);
     b.sortStatus = (unsigned long long *)take(8 * 256 * b.sortStatusTiles);
-    b.auxStatusTiles = (std::max(Ss, Ts) + fdzb::kSortTileHost - 1) / fdzb::kSortTileHost;
+    b.auxStatusTiles = fdzb::sort_tiles(std::max(Ss, Ts));
     b.auxStatus = (unsigned long long *)take(8 * 256 * b.auxStatusTiles);
     b.itemCapacity = (int)(Ss / 32 + (size_t)NB + (size_t)nf + 1);
     b.items = (int4 *)take(16 * (size_t)b.itemCapacity);
@@ -182,13 +184,51 @@ int ensure_arena(Engine &e, int nf, long long S, long long T, long long NB, long
     return FDZB_OK;
 }
 
-// Bytes of the frame table and of the counters up to what lies behind them.
-size_t frames_bytes(int nf) { return align_up(sizeof(fdzb::FrameDesc) * (size_t)nf, 256); }
 constexpr size_t kCountersBytes = (sizeof(fdzb::Counters) + 255) / 256 * 256;
+
+// Offsets in the pinned block of a launch of nf frames, those of the arena's:
+// frames, base offsets, and the counters and frame states it starts from.
+struct HostBlock {
+    size_t bases, counters, states, bytes;
+    explicit HostBlock(int nf)
+    {
+        bases = align_up(sizeof(fdzb::FrameDesc) * (size_t)nf, 256);
+        counters = bases + align_up(3 * sizeof(int) * (size_t)nf, 256);
+        states = counters + kCountersBytes;
+        bytes = states + sizeof(fdzb::FrameState) * (size_t)nf;
+    }
+};
+
+// f2o of the device code: floats in the order of their encodings.
+uint32_t ordered_bits(float f)
+{
+    uint32_t u;
+    std::memcpy(&u, &f, 4);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// The counters and frame states a launch starts from: zero, and the identities of
+// the bounds (maxima of light depths start at -1, the reference's reduction value,
+// K/Step2_1_*.inl:43, K/Step2_2_*.inl:40).
+void start_states(Engine &e, int nf)
+{
+    const HostBlock h(nf);
+    char *base = (char *)e.hFrames;
+    std::memset(base + h.counters, 0, h.bytes - h.counters);
+    fdzb::FrameState *st = (fdzb::FrameState *)(base + h.states);
+    for (int i = 0; i < nf; ++i) {
+        uint32_t *a = st[i].acc;
+        for (int k = 0; k < fdzb::ACC_COUNT; ++k) a[k] = ordered_bits(3.402823466e+38f);
+        for (int k : {fdzb::ACC_S_MAXA, fdzb::ACC_S_MAXB, fdzb::ACC_S_MAXW, fdzb::ACC_M_MAXA, fdzb::ACC_M_MAXB,
+                      fdzb::ACC_M_MAXW})
+            a[k] = ordered_bits(-3.402823466e+38f);
+        a[fdzb::ACC_SMAXW] = a[fdzb::ACC_TMAXW] = ordered_bits(-1.0f);
+    }
+}
 
 int ensure_host(Engine &e, int nf)
 {
-    e.hBases = (int *)((char *)e.hFrames + frames_bytes(nf));
+    e.hBases = (int *)((char *)e.hFrames + HostBlock(nf).bases);
     if (nf <= e.hCap) return FDZB_OK;
     if (e.pending) cudaStreamSynchronize(e.stream);
     drop_graph(e);
@@ -200,13 +240,13 @@ int ensure_host(Engine &e, int nf)
     e.hCounters = nullptr;
     e.hCap = 0;
     const int cap = std::max(nf, 1);
-    FDZB_CUDA(cudaMallocHost(&e.hFrames, frames_bytes(cap) + sizeof(int) * 3 * cap));
+    FDZB_CUDA(cudaMallocHost(&e.hFrames, HostBlock(cap).bytes));
     FDZB_CUDA(cudaMallocHost(&e.hCounters, kCountersBytes + sizeof(fdzb::FrameState) * cap));
     std::memset(e.hCounters, 0, kCountersBytes + sizeof(fdzb::FrameState) * cap);
     *e.hCounters = last;
     e.hStates = (fdzb::FrameState *)((char *)e.hCounters + kCountersBytes);
     e.hCap = cap;
-    e.hBases = (int *)((char *)e.hFrames + frames_bytes(nf));
+    e.hBases = (int *)((char *)e.hFrames + HostBlock(nf).bases);
     return FDZB_OK;
 }
 
@@ -291,7 +331,7 @@ cudaError_t enqueue_body(Engine &e, int nf)
     fdzb::DeviceBuffers &b = e.buf;
     cudaStream_t s = e.stream;
     cudaError_t err;
-    if ((err = cudaMemcpyAsync(b.frames, e.hFrames, frames_bytes(nf) + 3 * sizeof(int) * nf, cudaMemcpyHostToDevice, s)))
+    if ((err = cudaMemcpyAsync(b.frames, e.hFrames, HostBlock(nf).bytes, cudaMemcpyHostToDevice, s)))
         return err;
     // stage timing and debug copies want the stages one after the other
     const bool fork = !e.profile && !e.debug;
@@ -310,11 +350,10 @@ cudaError_t refresh_lookback(Engine &e)
     const auto where = std::make_tuple((const void *)b.sortStatus, b.sortStatusTiles + b.auxStatusTiles,
                                        (const void *)b.triScanStatus, b.totalTris, (const void *)b.epochWord);
     if (where != e.statusLayout || e.epochCount >= kEpochLimit) {
-        const size_t triTiles = ((size_t)std::max(b.totalTris, 1) + fdzb::kTriTileHost - 1) / fdzb::kTriTileHost;
         cudaError_t err;
         if ((err = cudaMemsetAsync(b.sortStatus, 0, 8 * 256 * b.sortStatusTiles, e.stream))) return err;
         if ((err = cudaMemsetAsync(b.auxStatus, 0, 8 * 256 * b.auxStatusTiles, e.stream))) return err;
-        if ((err = cudaMemsetAsync(b.triScanStatus, 0, 8 * triTiles, e.stream))) return err;
+        if ((err = cudaMemsetAsync(b.triScanStatus, 0, 8 * b.triScanTiles, e.stream))) return err;
         if ((err = cudaMemsetAsync(b.epochWord, 0, sizeof(uint32_t), e.stream))) return err;
         e.epochCount = 0;
         e.statusLayout = where;
@@ -427,6 +466,7 @@ int engine_enqueue(Engine &e)
         f.occChunk = s.occChunk;
         // the lane-per-pair schedule deals one item of 32 samples to a warp
         f.occItem = b.occVariant == 1 ? 32 : s.occItem;
+        if (i == 0) start_states(e, nf);
         e.hBases[i] = sb;
         e.hBases[nf + i] = tb;
         e.hBases[2 * nf + i] = bb;

@@ -105,7 +105,7 @@ struct Engine {
     bool lastFromGraph = false;
     long long graphCaptures = 0, graphReplays = 0;
     // Look-back tags: launches since the status words were last cleared (the
-    // device epoch word, advanced by k_init, holds the same count).  The words
+    // device epoch word, advanced by k_reduce, holds the same count).  The words
     // are cleared when the arena is laid out anew (they may then hold other
     // buffers' bytes) and before the count reaches kEpochLimit, so a tag never
     // wraps round to the tag of a stale word.

@@ -144,7 +144,7 @@ struct DeviceBuffers {
     // look-back words, epoch-tagged: [sortStatusTiles * 256] of the pair sort and
     // [auxStatusTiles * 256] of the sample and triangle sorts, which run beside it
     unsigned long long *sortStatus, *auxStatus;
-    size_t sortStatusTiles, auxStatusTiles;
+    size_t sortStatusTiles, auxStatusTiles, triScanTiles;
     int *sampleBases, *triBases, *binBases;     // [nframes] ascending global bases
     // occlusion work list
     int4 *items;                                // [itemCapacity]
@@ -163,7 +163,7 @@ struct DeviceBuffers {
     int countWork;                              // 1: the occlusion kernel that accumulates the work counters
     int rows16;                                 // 1: every grid of the launch has at most 16 rows of at most 31 columns
     uint32_t *epochWord;                        // launch sequence number (look-back tags), advanced
-                                                // on the device by k_init so graph replays stay fresh
+                                                // on the device by k_reduce so graph replays stay fresh
     // debug capture (nullptr unless enabled): pre-sort copies of the key/value arrays
     uint32_t *dbgKeys, *dbgVals, *dbgPKeys, *dbgPVals;
 };
@@ -198,7 +198,8 @@ cudaError_t run_move_model(float *vtx, int vstride, int V, const float m[16], cu
 #define FDZB_SORT_ITEMS 16
 #endif
 constexpr int kSortTileHost = 256 * FDZB_SORT_ITEMS;   // keys per radix-sort tile (fdzb_sort.cuh)
-constexpr int kTriTileHost = 64;      // triangles per pair-scan tile (the smaller of the two sizes)
+constexpr int kTriTileHost = 8;       // triangles per pair-scan tile (the smallest size)
+size_t sort_tiles(size_t keys);       // tiles a radix pass may cut `keys` keys into, at the most
 constexpr int kSortSlots = 3;        // radix sorts per launch: samples, pairs, triangles
 
 }  // namespace fdzb

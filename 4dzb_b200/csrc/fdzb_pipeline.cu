@@ -1,10 +1,10 @@
 // fdzb_pipeline.cu -- the B200 FDZB soft-shadow pipeline.
 //
 // Stage map (reference kernels in 4DZB/FDZB_Soft_Shadow/cuda/, "K/"):
-//   k_init        clears per-launch bin state, counters and digit histograms
 //   k_reduce      k1+k2+k3+k4 fused: one pass over samples (pos+normal, 128-bit
 //                 loads) and vertices computes the far-plane depth maxima and the
-//                 sample / vertex rectangle bounds (K/Step2_1_*, K/Step2_2_*); the
+//                 sample / vertex rectangle bounds (K/Step2_1_*, K/Step2_2_*), beside
+//                 the clearing of the bins, segments and digit histograms; the
 //                 frame's last block plans it: light plane, far plane f,
 //                 sub-constant, bin factor (K/Step2_3_defineFDbuffer.inl:5-111)
 //   k_tri_setup   per-triangle cull + footprint AABB + 64-byte record
@@ -40,48 +40,30 @@ __device__ __forceinline__ f3 load_vertex(const FrameDesc &fr, int v)
     return fr.hasXform ? transform_point(fr.xform, q) : q;
 }
 
-// ---------------------------------------------------------------------------
-// k_init: empty bin statistics (K/Step3_bindSampleToBin.inl:83-84) and cleared
-// segment tables (K/binRaster.inl:39-40, 52-53).
-// ---------------------------------------------------------------------------
-__global__ void k_init(FrameState *states, int nframes, uint32_t *binStat, int32_t *bss,
-                       int32_t *bse, int32_t *bts, int32_t *bte, int totalBins, uint32_t *epochWord,
-                       Counters *counters, uint32_t *sortHist)
+// What a launch clears: the digit histograms, the empty bin statistics
+// (K/Step3_bindSampleToBin.inl:83-84) and the segment tables
+// (K/binRaster.inl:39-40, 52-53).
+struct ClearTargets {
+    uint32_t *binStat;
+    int32_t *bss, *bse, *bts, *bte;
+    int totalBins;
+    uint32_t *epochWord, *sortHist;
+};
+
+__device__ __forceinline__ void clear_launch(const ClearTargets &c, int gid, int stride)
 {
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid == 0) *epochWord += 1u;  // launch number: look-back tags of this launch
-    const int stride = gridDim.x * blockDim.x;
-    static_assert(sizeof(Counters) % sizeof(uint32_t) == 0, "counters cleared word by word");
-    for (int i = gid; i < (int)(sizeof(Counters) / sizeof(uint32_t)); i += stride)
-        reinterpret_cast<uint32_t *>(counters)[i] = 0u;
-    for (int i = gid; i < 4 * kSortSlots * kRadix; i += stride) sortHist[i] = 0u;
+    if (gid == 0) *c.epochWord += 1u;  // launch number: look-back tags of this launch
+    for (int i = gid; i < 4 * kSortSlots * kRadix; i += stride) c.sortHist[i] = 0u;
     const uint32_t neg = f2o(-kF32Max), pos = f2o(kF32Max);
-    for (int b = gid; b < totalBins; b += stride) {
-        uint4 s0 = make_uint4(neg, neg, neg, pos);
-        uint4 s1 = make_uint4(pos, 0u, 0u, 0u);
-        reinterpret_cast<uint4 *>(binStat)[2 * b] = s0;
-        reinterpret_cast<uint4 *>(binStat)[2 * b + 1] = s1;
-        bts[b] = kSegAbsent;   // segment bounds: lowered / raised by the sorts' last passes
-        bte[b] = 0;
+    for (int b = gid; b < c.totalBins; b += stride) {
+        reinterpret_cast<uint4 *>(c.binStat)[2 * b] = make_uint4(neg, neg, neg, pos);
+        reinterpret_cast<uint4 *>(c.binStat)[2 * b + 1] = make_uint4(pos, 0u, 0u, 0u);
+        c.bts[b] = kSegAbsent;   // segment bounds: lowered / raised by the sorts' last passes
+        c.bte[b] = 0;
     }
-    for (int b = gid; b <= totalBins; b += stride) {
-        bss[b] = kSegAbsent;
-        bse[b] = 0;
-    }
-    for (int f = gid; f < nframes; f += stride) {
-        FrameState &s = states[f];
-        s.acc[ACC_SMAXW] = f2o(-1.0f);  // thrust::reduce init value (K/Step2_1_*.inl:43)
-        s.acc[ACC_TMAXW] = f2o(-1.0f);  // (K/Step2_2_*.inl:40)
-        s.acc[ACC_S_MINU] = pos; s.acc[ACC_S_MINV] = pos; s.acc[ACC_S_MINW] = pos;
-        s.acc[ACC_S_MAXA] = neg; s.acc[ACC_S_MAXB] = neg; s.acc[ACC_S_MAXW] = neg;
-        s.acc[ACC_M_MINU] = pos; s.acc[ACC_M_MINV] = pos; s.acc[ACC_M_MINW] = pos;
-        s.acc[ACC_M_MAXA] = neg; s.acc[ACC_M_MAXB] = neg; s.acc[ACC_M_MAXW] = neg;
-        s.nFront = 0;
-        s.state = 0;
-        s.nValidTris = 0;
-        s.nValidSamples = 0;
-        s.quirkKeyRange = 0;
-        s.arrived = 0;
+    for (int b = gid; b <= c.totalBins; b += stride) {
+        c.bss[b] = kSegAbsent;
+        c.bse[b] = 0;
     }
 }
 
@@ -144,7 +126,9 @@ __device__ void plan_frame(const FrameDesc &fr, FrameState &st)
 // the subtraction (sub = RF/f needs f first): fl(x - sub) is monotone in x, so
 // max_i fl(a_i - sub) == fl(max_i a_i - sub) exactly.
 // Vertex part: k2 (max depth) and k4 (vertex rectangle bounds).  The frame's
-// last block plans it (a launch of its own before: 3 us and a gap).
+// last block plans it.  A launch's clears are done here too: its counters and frame
+// states arrive with the frame table.  (Launches of their own before: 3 us and a
+// gap each.)
 // ---------------------------------------------------------------------------
 constexpr int kReduceThreads = 256;
 
@@ -158,8 +142,10 @@ __device__ __forceinline__ void acc_min(uint32_t &a, float v)
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
-    k_reduce(const FrameDesc *__restrict__ frames, FrameState *states)
+    k_reduce(const FrameDesc *__restrict__ frames, FrameState *states, ClearTargets clear)
 {
+    clear_launch(clear, ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
+                 gridDim.x * gridDim.y * gridDim.z * blockDim.x);
     const FrameDesc &fr = frames[blockIdx.y];
     FrameState &st = states[blockIdx.y];
     const float *M = fr.light.mat;
@@ -535,7 +521,7 @@ __global__ void __launch_bounds__(256)
 // (:184-202) with the counting predicate used for both passes.
 // ---------------------------------------------------------------------------
 constexpr int kTriThreads = 256;
-constexpr int kTriTile = 64;   // triangles per pair-scan tile (launches of up to kTriSmallLaunch triangles)
+constexpr int kTriTiny = 32;   // triangles per SM up to which a tile has 8 (a triangle a warp)
 constexpr int kTriSmallLaunch = 1 << 20;
 // Look-back status word of a triangle tile: [63:32] launch epoch, [31:30] flag,
 // [29:0] pair count (the pair capacity stays below 2^30).
@@ -591,7 +577,8 @@ __device__ __forceinline__ bool stat_accepts(uint4 s, uint32_t s4, const TriBins
 // bin << triBits | triangle.
 __device__ __forceinline__ int sweep_bins(const uint32_t *__restrict__ binStat, const TriBins &c, int bb, int l2,
                                           int lane, uint32_t *__restrict__ pkeys, uint32_t *__restrict__ pvals,
-                                          unsigned long long pos, int capacity, int g, bool write, int triBits)
+                                          unsigned long long pos, int capacity, int g, bool write, int triBits,
+                                          uint32_t *hist, int passes)
 {
     const int w = c.cex - c.cbx, h = c.cey - c.cby;
     if (w <= 0 || h <= 0) return 0;
@@ -631,15 +618,27 @@ __device__ __forceinline__ int sweep_bins(const uint32_t *__restrict__ binStat, 
             ok = stat_accepts(sc, sc4, c);
         }
         const unsigned m = __ballot_sync(kFullWarp, ok);
-        if (write && ok) {
+        if (write && m) {
             const unsigned long long p = pos + (unsigned long long)total + (unsigned)__popc(m & lanemask_lt());
-            if (p < (unsigned long long)capacity) {
+            const bool put = ok && p < (unsigned long long)capacity;
+            if (put) {
                 if (triBits) {
                     pkeys[p] = ((uint32_t)gb << triBits) | (uint32_t)g;
                 } else {
                     pkeys[p] = (uint32_t)gb;
                     pvals[p] = (uint32_t)g;
                 }
+                atomicAdd(&hist[gb & 255], 1u);
+            }
+            // digit counts for the pair sort: the low digits of a row of bins differ,
+            // the higher ones are mostly the same, one count for all lanes that have
+            // the first one's
+            for (int q = 1; q < passes; ++q) {
+                const int d = (gb >> (8 * q)) & 255;
+                const int d0 = __shfl_sync(kFullWarp, d, __ffs(m) - 1);
+                const unsigned same = __ballot_sync(kFullWarp, put && d == d0);
+                if (lane == 0 && same) atomicAdd(&hist[q * kRadix + d0], (uint32_t)__popc(same));
+                if (put && d != d0) atomicAdd(&hist[q * kRadix + d], 1u);
             }
         }
         total += __popc(m);
@@ -667,7 +666,8 @@ __global__ void __launch_bounds__(kTriThreads, 4)
                 const float4 *__restrict__ rec, const uint32_t *__restrict__ binStat,
                 int32_t *__restrict__ triCount, unsigned long long *scanStatus, const uint32_t *epochWord,
                 uint32_t *__restrict__ pkeys, uint32_t *__restrict__ pvals, int capacity,
-                const uint32_t *__restrict__ order, int triBits, Counters *ctr)
+                const uint32_t *__restrict__ order, int triBits, int passes, uint32_t *__restrict__ sortHist,
+                Counters *ctr)
 {
     constexpr int WARPS = kTriThreads / 32;
     constexpr int TPW = TILE / WARPS;   // triangles per warp and tile
@@ -676,9 +676,11 @@ __global__ void __launch_bounds__(kTriThreads, 4)
     __shared__ int s_cnt[TILE];
     __shared__ unsigned long long s_wsum[WARPS];
     __shared__ unsigned long long s_excl;
+    __shared__ uint32_t s_hist[4 * kRadix];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ntiles = (totalTris + TILE - 1) / TILE;
     const uint32_t epoch = *epochWord;
+    for (int i = tid; i < passes * kRadix; i += kTriThreads) s_hist[i] = 0;
     for (;;) {
         __syncthreads();
         if (tid == 0) s_tile = atomicAdd(&ctr->triTileCounter, 1);
@@ -733,7 +735,8 @@ __global__ void __launch_bounds__(kTriThreads, 4)
             take(j, c, g, bb, l2);
             int cnt = 0;
             if (g >= 0) {
-                if (c.any) cnt = sweep_bins(binStat, c, bb, l2, lane, pkeys, pvals, 0, capacity, g, false, triBits);
+                if (c.any) cnt = sweep_bins(binStat, c, bb, l2, lane, pkeys, pvals, 0, capacity, g, false, triBits,
+                                             nullptr, 0);
                 if (lane == 0) triCount[g] = cnt;
             }
             if (lane == 0) s_cnt[k] = cnt;
@@ -758,39 +761,45 @@ __global__ void __launch_bounds__(kTriThreads, 4)
         __syncthreads();
         if (tid < TILE)
             s_cnt[tid] = (int)min(mine_excl, (unsigned long long)0x7fffffff);   // now: exclusive offset in the tile
-        if (tid == 0) {
+        if (warp == 0) {
+            // 32 tiles back at a time, a lane each
             unsigned long long excl = 0;
             unsigned long long *my = scanStatus + tile;
             const unsigned long long ep = (unsigned long long)epoch << 32;
             const unsigned long long tot = total > kScanMask ? kScanMask : total;
-            if (tile == 0) {
-                st_volatile_u64(my, ep | kScanPrefix | tot);
-            } else {
-                st_volatile_u64(my, ep | kScanAgg | tot);
-                int t = tile - 1;
-                unsigned spins = 0;
-                while (t >= 0) {
-                    const unsigned long long s = ld_volatile_u64(scanStatus + t);
-                    const unsigned long long flag = ((s >> 32) == epoch) ? (s & 0xC0000000ull) : 0ull;
-                    if (flag == 0) {
-                        if (++spins > kSpinLimit) {
-                            atomicOr(&ctr->errorFlags, (int)ERR_LOOKBACK_TIMEOUT);
-                            break;
-                        }
-                        continue;
-                    }
-                    excl += s & kScanMask;
-                    if (flag == kScanPrefix) break;
-                    --t;
+            if (lane == 0) st_volatile_u64(my, ep | (tile == 0 ? kScanPrefix : kScanAgg) | tot);
+            unsigned spins = 0;
+            for (int t = tile - 1; t >= 0;) {
+                const unsigned long long st = t - lane >= 0 ? ld_volatile_u64(scanStatus + (t - lane)) : 0ull;
+                const unsigned long long flag = (t - lane >= 0 && (st >> 32) == epoch) ? (st & 0xC0000000ull) : 0ull;
+                const unsigned none = __ballot_sync(kFullWarp, flag == 0);
+                const unsigned prefix = __ballot_sync(kFullWarp, flag == kScanPrefix);
+                // the published tiles before the first gap, up to the first prefix
+                int take = none ? __ffs(none) - 1 : 32;
+                const bool done = prefix && __ffs(prefix) <= take;
+                if (done) take = __ffs(prefix);
+                unsigned long long v = lane < take ? st & kScanMask : 0ull;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullWarp, v, o);
+                excl += v;
+                if (done) break;
+                t -= take;
+                if (take == 0 && ++spins > kSpinLimit) {
+                    if (lane == 0) atomicOr(&ctr->errorFlags, (int)ERR_LOOKBACK_TIMEOUT);
+                    break;
                 }
+            }
+            if (lane == 0 && tile > 0) {
                 const unsigned long long inc = excl + total > kScanMask ? kScanMask : excl + total;
                 st_volatile_u64(my, ep | kScanPrefix | inc);
             }
-            s_excl = excl;
-            if (tile == ntiles - 1) {
-                const unsigned long long all = excl + total;
-                ctr->pairCount = (int)(all > 0x7fffffffull ? 0x7fffffffull : all);
-                if (all > (unsigned long long)capacity) ctr->pairOverflow = 1;
+            if (lane == 0) {
+                s_excl = excl;
+                if (tile == ntiles - 1) {
+                    const unsigned long long all = excl + total;
+                    ctr->pairCount = (int)(all > 0x7fffffffull ? 0x7fffffffull : all);
+                    if (all > (unsigned long long)capacity) ctr->pairOverflow = 1;
+                }
             }
         }
         __syncthreads();
@@ -803,9 +812,10 @@ __global__ void __launch_bounds__(kTriThreads, 4)
             take(j, c, g, bb, l2);
             if (g < 0 || !c.any) continue;
             sweep_bins(binStat, c, bb, l2, lane, pkeys, pvals, tileBase + (unsigned long long)s_cnt[k], capacity, g,
-                       true, triBits);
+                       true, triBits, s_hist, passes);
         }
     }
+    flush_hist(s_hist, passes * kRadix, sortHist);
 }
 
 // ---------------------------------------------------------------------------
@@ -847,7 +857,6 @@ cudaError_t run_move_model(float *vtx, int vstride, int V, const float m[16], cu
 // Host driver.
 // ---------------------------------------------------------------------------
 static_assert(kSortTileHost == kSortTile, "sort tile mismatch");
-static_assert(kTriTileHost == kTriTile, "pair-scan tile mismatch");
 
 int sort_passes_for(long long keyRangeExclusive)
 {
@@ -875,16 +884,22 @@ static int grid_for(long long n, int threads, int cap)
 #define FDZB_SORTK_MINBLOCKS 4
 #endif
 constexpr int kKeysItems = FDZB_SORTK_ITEMS, kKeysMinBlocks = FDZB_SORTK_MINBLOCKS;
-constexpr int kKeysTile = kSortThreads * kKeysItems;
-static_assert(kKeysTile >= kSortTile, "the look-back status array is sized for tiles of kSortTile keys");
+static_assert(kKeysItems >= kSortItems && kKeysItems % 4 == 0 && kSortItems % 4 == 0,
+              "the look-back status array is sized for tiles of kSortItems keys a thread, or a quarter of them");
+
+size_t sort_tiles(size_t keys)
+{
+    const size_t full = (keys + kSortTile - 1) / kSortTile;
+    const size_t few = ((keys < (size_t)kSmallSort ? keys : (size_t)kSmallSort) + kSortTile / 4 - 1) / (kSortTile / 4);
+    return full > few ? full : few;
+}
 
 // Sorts (kA, vA) with kB/vB as ping-pong buffers; `slot` selects the histogram
 // and ticket block (0 samples, 1 pairs, 2 triangles).  Pass p uses tag
 // 16*launch + 4*slot + p and the key's bits [shift0 + 8p, shift0 + 8p + 8).
 // vA == nullptr: keys alone.  With segStart/segEnd the last pass also writes
 // the bounds of the segments key >> segShift (nslots of them; K/binRaster.inl:5-33).
-// The digit counts are in the slot's histogram already where the keys' producer
-// made them (slots 0 and 2); the pair sort's are counted here.
+// The digit counts are in the slot's histogram already: the keys' producer made them.
 static void run_sort(const DeviceBuffers &b, int slot, uint32_t *kA, uint32_t *vA, uint32_t *kB,
                      uint32_t *vB, const int *n_dev, int n_static, int cap, int passes, int sm,
                      cudaStream_t s, int shift0 = 0, int32_t *segStart = nullptr, int32_t *segEnd = nullptr,
@@ -892,13 +907,10 @@ static void run_sort(const DeviceBuffers &b, int slot, uint32_t *kA, uint32_t *v
 {
     uint32_t *hist = b.sortHist + slot * 4 * kRadix;
     unsigned long long *status = slot == 1 ? b.sortStatus : b.auxStatus;
-    if (slot == 1) k_radix_hist<<<grid_for(cap, kSortThreads, sm * 4), kSortThreads, 0, s>>>(kA, n_dev, n_static,
-                                                                              cap, passes, shift0, hist);
     uint32_t *ki = kA, *vi = vA, *ko = kB, *vo = vB;
-    const long long tiles = ((long long)cap + kSortTile - 1) / kSortTile;
+    const long long tiles = (long long)sort_tiles((size_t)cap);
     const int passGrid = grid_for(tiles * kSortThreads, kSortThreads, sm * 4);
-    const long long keysTiles = ((long long)cap + kKeysTile - 1) / kKeysTile;
-    const int keysGrid = grid_for(keysTiles * kSortThreads, kSortThreads, sm * kKeysMinBlocks);
+    const int keysGrid = grid_for(tiles * kSortThreads, kSortThreads, sm * kKeysMinBlocks);
     for (int p = 0; p < passes; ++p) {
         const bool seg = segStart && p == passes - 1;
 #define FDZB_PASS_ARGS(VI, VO)                                                                               \
@@ -947,12 +959,11 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     int nl = 0;
     if (ev) cudaEventRecord(ev[STAGE_SETUP], s);
     // (a) samples, vertices, triangles
-    k_init<<<grid_for(b.totalBins + 1, 256, sm * 8), 256, 0, s>>>(
-        b.states, nf, b.binStat, b.binSampleStart, b.binSampleEnd, b.binTriStart, b.binTriEnd, b.totalBins,
-        b.epochWord, b.counters, b.sortHist);
     {
         const int gx = grid_for(maxS > maxV ? maxS : maxV, kReduceThreads, sm * 4);
-        k_reduce<<<dim3(gx, nf, 2), kReduceThreads, 0, s>>>(b.frames, b.states);
+        k_reduce<<<dim3(gx, nf, 2), kReduceThreads, 0, s>>>(
+            b.frames, b.states, {b.binStat, b.binSampleStart, b.binSampleEnd, b.binTriStart, b.binTriEnd, b.totalBins,
+                                 b.epochWord, b.sortHist});
     }
     const bool ordered = b.depthBits > 0 && b.totalTris > 0;
     k_tri_setup<<<dim3(grid_for(maxT, 256, sm * 8), nf), 256, 0, s>>>(
@@ -995,7 +1006,7 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
         sample_sort();
     }
     uint32_t *sv = (b.samplePasses & 1) ? b.valsB : b.valsA;
-    nl += 4 + b.samplePasses;
+    nl += 3 + b.samplePasses;
     // (a) triangle/bin pairs, in the coverage order when one is asked for
     if (ev) cudaEventRecord(ev[STAGE_TRI_PAIRS], s);
     const uint32_t *order = nullptr;
@@ -1011,20 +1022,14 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
         // above, tiles of 256 (64 frames, 8.9M triangles: 7.1 ms against 8.4
         // ms with tiles of 64).  Up to 8 blocks per SM: the sweeps wait on
         // bin-statistics loads, so more resident warps hide more of that latency.
-        const bool small = b.totalTris <= kTriSmallLaunch;
-        const int tile = small ? kTriTile : 256;
+        const int tile = b.totalTris <= kTriTiny * sm ? 8 : b.totalTris <= kTriSmallLaunch ? 64 : 256;
         const int tiles = (b.totalTris + tile - 1) / tile;
         const int grid = tiles < sm * 8 ? (tiles > 0 ? tiles : 1) : sm * 8;
-        if (small)
-            k_tri_pairs<kTriTile><<<grid, kTriThreads, 0, s>>>(b.frames, b.states, b.triBases, nf, b.totalTris,
-                                                               b.triRec, b.binStat, b.triCount, b.triScanStatus,
-                                                               b.epochWord, b.pkeysA, b.pvalsA, b.pairCapacity,
-                                                               order, b.pairTriBits, b.counters);
-        else
-            k_tri_pairs<256><<<grid, kTriThreads, 0, s>>>(b.frames, b.states, b.triBases, nf, b.totalTris,
-                                                          b.triRec, b.binStat, b.triCount, b.triScanStatus,
-                                                          b.epochWord, b.pkeysA, b.pvalsA, b.pairCapacity,
-                                                          order, b.pairTriBits, b.counters);
+        auto pairs = tile == 8 ? k_tri_pairs<8> : tile == 64 ? k_tri_pairs<64> : k_tri_pairs<256>;
+        pairs<<<grid, kTriThreads, 0, s>>>(b.frames, b.states, b.triBases, nf, b.totalTris, b.triRec, b.binStat,
+                                           b.triCount, b.triScanStatus, b.epochWord, b.pkeysA, b.pvalsA,
+                                           b.pairCapacity, order, b.pairTriBits, b.pairPasses,
+                                           b.sortHist + 4 * kRadix, b.counters);
         nl += 1;
     }
     if (b.dbgPKeys) {
@@ -1043,7 +1048,7 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     uint32_t *pk = (b.pairPasses & 1) ? b.pkeysB : b.pkeysA;
     uint32_t *pv = packed ? pk : ((b.pairPasses & 1) ? b.pvalsB : b.pvalsA);
     const uint32_t triMask = packed ? (1u << b.pairTriBits) - 1u : 0xFFFFFFFFu;
-    nl += 1 + b.pairPasses;
+    nl += b.pairPasses;
     // (c) + (d) occlusion and shading
     if (ev) cudaEventRecord(ev[STAGE_OCCLUSION], s);
     if (fork) cudaStreamWaitEvent(s, fork->samples, 0);
@@ -1349,6 +1354,7 @@ namespace {
 
 constexpr int kNoAllocMaxPairs = 1 << 20;   // FDZB_NOALLOC_SORT_MAX_PAIRS
 constexpr int kNoAllocTiles = (kNoAllocMaxPairs + kSortTile - 1) / kSortTile;
+static_assert(kNoAllocTiles >= kSmallSort / (kSortTile / 4), "tiles of a sort of few keys");
 constexpr size_t kNoAllocKeysOff = 0;
 constexpr size_t kNoAllocValsOff = kNoAllocKeysOff + 4ull * kNoAllocMaxPairs;
 constexpr size_t kNoAllocHistOff = kNoAllocValsOff + 4ull * kNoAllocMaxPairs;
@@ -1424,7 +1430,7 @@ extern "C" int fdzb_sort_pairs_noalloc(const uint32_t *d_keys_in, const uint32_t
     int *tickets = (int *)(base + kNoAllocTicketOff);
     int *err = (int *)(base + kNoAllocErrOff);
     unsigned long long *status = (unsigned long long *)(base + kNoAllocStatusOff);
-    const long long tiles = ((long long)n + kSortTile - 1) / kSortTile;
+    const long long tiles = (long long)sort_tiles((size_t)n);
     // histogram, tickets, error word and the look-back words of the tiles in
     // use start at zero every call (one contiguous range, at most 0.5 MiB)
     e = cudaMemsetAsync(hist, 0, kNoAllocStatusOff - kNoAllocHistOff + 8ull * kRadix * (size_t)tiles, s);

@@ -3,10 +3,9 @@
 // Replaces the reference's thrust::sort_by_key calls
 // (K/Step3_bindSampleToBin.inl:125-127, K/Step4_RasterizeTriangleToBin.inl:221-223):
 // same result (keys ascending, equal keys in input order), one-sweep design:
-//   1. one histogram counts the 8-bit digits of every pass at once (shared-memory
-//      digit histograms, one global atomic per digit per block): made by the kernel
-//      that writes the keys, or a pass of its own where their number is not known
-//      before (the pairs);
+//   1. the 8-bit digits of every pass are counted at once (shared-memory digit
+//      histograms, one global atomic per digit and block) by the kernel that writes
+//      the keys, or by k_radix_hist for keys that come from elsewhere;
 //   2. one scatter pass per digit: each CTA takes the next tile ticket, ranks its
 //      keys with warp match/popc against per-warp shared histograms, publishes its
 //      per-digit tile count, and finds its global offsets by a decoupled look-back
@@ -27,6 +26,11 @@ constexpr int kSortThreads = 256;                      // = kRadix: thread d han
 constexpr int kSortItems = FDZB_SORT_ITEMS;
 constexpr int kSortTile = kSortThreads * kSortItems;   // keys per tile
 constexpr int kRadix = 256;
+// Keys of a sort that is cut into tiles of a quarter of the items: up to here
+// the full tiles leave SMs without one, and a thread's serial share of a tile is
+// most of a pass.
+constexpr int kSmallSort = 1 << 17;
+constexpr int kLookBack = 4;                           // predecessors a thread asks for at once
 // Look-back status word: [63:32] launch epoch, [31:30] flag, [29:0] count.  A
 // word whose epoch is not the current one reads as "not yet published", so the
 // status array never needs clearing between launches or passes.
@@ -80,19 +84,21 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
                  uint32_t nslots = 0)
 {
     constexpr int WARPS = kSortThreads / 32;
-    constexpr int TILE = kSortThreads * ITEMS;
+    constexpr int TILE_MAX = kSortThreads * ITEMS;
     __shared__ uint32_t s_start[kRadix];
     __shared__ uint32_t s_whist[WARPS][kRadix];
     __shared__ uint32_t s_base[kRadix];
     __shared__ uint32_t s_tstart[kRadix];
     __shared__ uint32_t s_scan[WARPS];
-    __shared__ uint32_t s_k[TILE];
-    __shared__ uint32_t s_v[KV ? TILE : 1];
+    __shared__ uint32_t s_k[TILE_MAX];
+    __shared__ uint32_t s_v[KV ? TILE_MAX : 1];
     __shared__ int s_tile;
 
     const int n = sort_count(n_dev, n_static, cap);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // look-back tag of this pass: 16 x (launch number, a device word that k_init
+    const int nItems = n <= kSmallSort ? ITEMS / 4 : ITEMS;   // keys a thread, of this launch
+    const int TILE = kSortThreads * nItems;
+    // look-back tag of this pass: 16 x (launch number, a device word that k_reduce
     // advances, so graph replays get fresh tags) + 4 x sort slot + pass
     const uint32_t epoch = (epochWord ? *epochWord * 16u : 0u) + epochLo;
 
@@ -121,17 +127,18 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         if ((long long)tile * TILE >= n) break;
         const int tileN = min(TILE, n - tile * TILE);
 
-        const int base = tile * TILE + warp * (ITEMS * 32);
+        const int base = tile * TILE + warp * (nItems * 32);
         uint32_t k[ITEMS], v[ITEMS], rk[ITEMS];
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
             const int idx = base + i * 32 + lane;
-            const bool ok = idx < n;
+            const bool ok = i < nItems && idx < n;
             k[i] = ok ? kin[idx] : 0u;
             v[i] = (KV && ok) ? vin[idx] : 0u;
         }
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
+            if (i >= nItems) break;
             const int idx = base + i * 32 + lane;
             const bool ok = idx < n;
             const uint32_t d = ok ? ((k[i] >> shift) & 255u) : 256u;
@@ -177,18 +184,30 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
             int t = tile - 1;
             unsigned spins = 0;
             while (t >= 0) {
-                const unsigned long long s = ld_volatile_u64(status + (size_t)t * kRadix + tid);
-                const unsigned long long flag = ((s >> 32) == epoch) ? (s & 0xC0000000ull) : 0ull;
-                if (flag == 0) {
-                    if (++spins > kSpinLimit) {
-                        atomicOr(err, (int)ERR_LOOKBACK_TIMEOUT);
-                        break;
+                // the words of the next tiles back in flight together; taken in
+                // order up to the first one that is not published yet
+                unsigned long long s[kLookBack];
+#pragma unroll
+                for (int j = 0; j < kLookBack; ++j)
+                    s[j] = t - j >= 0 ? ld_volatile_u64(status + (size_t)(t - j) * kRadix + tid) : 0ull;
+                int taken = 0;
+                bool done = false, open = true;
+#pragma unroll
+                for (int j = 0; j < kLookBack; ++j) {
+                    const unsigned long long flag = ((s[j] >> 32) == epoch) ? (s[j] & 0xC0000000ull) : 0ull;
+                    open = open && !done && t - j >= 0 && flag != 0;
+                    if (open) {
+                        excl += (uint32_t)(s[j] & kStatMask);
+                        done = flag == kStatPrefix;
+                        taken = j + 1;
                     }
-                    continue;
                 }
-                excl += (uint32_t)(s & kStatMask);
-                if (flag == kStatPrefix) break;
-                --t;
+                if (done) break;
+                t -= taken;
+                if (taken == 0 && ++spins > kSpinLimit) {
+                    atomicOr(err, (int)ERR_LOOKBACK_TIMEOUT);
+                    break;
+                }
             }
             st_volatile_u64(my, ep | kStatPrefix | (excl + run));
         }
@@ -199,6 +218,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         // reorder the tile by digit in shared memory (stable)
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
+            if (i >= nItems) break;
             const int idx = base + i * 32 + lane;
             if (idx < n) {
                 const uint32_t d = (k[i] >> shift) & 255u;
