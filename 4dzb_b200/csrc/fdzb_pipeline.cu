@@ -1076,18 +1076,17 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     // team: an item for each block at the most (an item is 32 samples or more of
     // one bin).  The counting forms and those without the cull keep a warp per item.
     const long long mostItems = b.totalSamples / 32 + (b.totalBins < b.totalSamples ? b.totalBins : b.totalSamples);
-    const bool team = b.openBox && !b.countWork && mostItems <= (b.wide ? g64 : g32);
+    const bool team = b.openBox && !b.countWork && mostItems <= g32;
 #define FDZB_OCC_FORMS(RT, ROWS, G, T)                                                                        \
     do {                                                                                                     \
-        if (team && b.depthPlane)                                                                            \
-            k_occlusion<RT, 1, 1, 0, ROWS, 1><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
-        else if (team)                                                                                       \
-            k_occlusion<RT, 0, 1, 0, ROWS, 1><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
-        else if (b.depthPlane && b.openBox) FDZB_OCC(RT, 1, 1, ROWS, G, T);                                        \
+        if (b.depthPlane && b.openBox) FDZB_OCC(RT, 1, 1, ROWS, G, T);                                        \
         else if (b.depthPlane) FDZB_OCC(RT, 1, 0, ROWS, G, T);                                                \
         else if (b.openBox) FDZB_OCC(RT, 0, 1, ROWS, G, T);                                                   \
         else FDZB_OCC(RT, 0, 0, ROWS, G, T);                                                                  \
     } while (0)
+#define FDZB_OCC_TEAM(DP, ROWS)                                                                               \
+    k_occlusion<uint32_t, DP, 1, 0, ROWS, 1><<<g32, kOccThreads, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, \
+                                                                        b.totalBins, nf)
 #define FDZB_RAYCAST(RT, G, T)                                                                                \
     do {                                                                                                     \
         if (b.countWork) k_raycast<RT, 1><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.totalTris, b.totalBins, nf);      \
@@ -1097,15 +1096,22 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
         if (b.wide) FDZB_RAYCAST(u64, g64, t64);
         else FDZB_RAYCAST(uint32_t, g32, kOccThreads);
     } else if (b.wide) {
-        FDZB_OCC_FORMS(u64, 64, g64, t64);
+        FDZB_OCC_FORMS(u64, 64, g64, t64);   // a warp per block, no teams
     } else if (b.occVariant == 1) {
         k_occlusion_pairs<<<sm * FDZB_OCC2_MINBLOCKS, kOccThreads, 0, s>>>(FDZB_OCC_LISTS, b.totalTris, b.totalBins, nf);
+    } else if (team && b.depthPlane) {
+        if (b.rows16) FDZB_OCC_TEAM(1, 16);
+        else FDZB_OCC_TEAM(1, 32);
+    } else if (team) {
+        if (b.rows16) FDZB_OCC_TEAM(0, 16);
+        else FDZB_OCC_TEAM(0, 32);
     } else if (b.rows16) {
         FDZB_OCC_FORMS(uint32_t, 16, g32, kOccThreads);
     } else {
         FDZB_OCC_FORMS(uint32_t, 32, g32, kOccThreads);
     }
 #undef FDZB_RAYCAST
+#undef FDZB_OCC_TEAM
 #undef FDZB_OCC_FORMS
 #undef FDZB_OCC
 #undef FDZB_OCC_LISTS

@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
     (61, 37, 1, 8, 8, 1, 32, 32, 0),         # one triangle for four warps
     (61, 37, 3, 16, 16, 1, 32, 128, 0),
     (61, 37, 130, 16, 32, 2, 32, 32, 0),     # 32-row masks, a last chunk of few
-    (61, 37, 700, 33, 33, 1, 8, 128, 0),     # 64-bit rows, two warps a block, many rounds
+    (61, 37, 700, 33, 33, 1, 8, 128, 0),     # 64-bit rows: a warp per block, no team
     (96, 60, 500, 8, 8, 8, 8, 32, 0),
     (96, 60, 4000, 17, 5, 8, 32, 64, 2000),   # several triangle passes
     (208, 150, 300, 8, 8, 8, 32, 32, 0),     # the two sides of the rule: 975 + 64 items at most
