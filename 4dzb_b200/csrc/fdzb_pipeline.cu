@@ -251,17 +251,23 @@ __global__ void __launch_bounds__(kReduceThreads)
 // the pair counter's skip test rejects them exactly as K/Step4_*.inl:41 does.
 // ---------------------------------------------------------------------------
 // Coverage-order bucket of a triangle (the key of the triangle sort): the triangle's
-// angular size seen from below, world area / (f - minz)^2 with f - minz the
-// light-depth distance from the far plane (about the receivers' depth) to the
-// triangle's vertex nearest the light, as a log-scale bucket; the largest
-// come first.  A sample's mask is the OR over its bin's triangles, so the order
-// changes only how soon its light rows fill (the early-out), never the result.
-__device__ __forceinline__ uint32_t coverage_bucket(f3 v0, f3 v1, f3 v2, float minz, float f, int depthBits)
+// solid angle seen from the receivers, its area across the line to the light's
+// centre / (f - minz)^2 with f - minz the light-depth distance from the far plane
+// (about the receivers' depth) to the triangle's vertex nearest the light, as a
+// log-scale bucket; the largest come first.  A sample's mask is the OR over its
+// bin's triangles, so the order changes only how soon its light rows fill (the
+// early-out), never the result.  Against the whole area, which puts triangles seen
+// edge-on first: 1920 x 1080, 200k triangles: 112.7M -> 88.7M pair tests, 3.92 ->
+// 3.07 ms; a projection from each bin's own centre saves no more.
+__device__ __forceinline__ uint32_t coverage_bucket(f3 v0, f3 v1, f3 v2, f3 light, float minz, float f, int depthBits)
 {
     const float ax = v1.x - v0.x, ay = v1.y - v0.y, az = v1.z - v0.z;
     const float bx = v2.x - v0.x, by = v2.y - v0.y, bz = v2.z - v0.z;
     const float cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
-    const float area2 = fmaxf(sqrtf(cx * cx + cy * cy + cz * cz), 1e-30f);
+    // towards the light's centre, from the triangle's
+    const float tx = light.x - (v0.x + v1.x + v2.x) * (1.0f / 3.0f), ty = light.y - (v0.y + v1.y + v2.y) * (1.0f / 3.0f),
+                tz = light.z - (v0.z + v1.z + v2.z) * (1.0f / 3.0f);
+    const float area2 = fmaxf(fabsf(cx * tx + cy * ty + cz * tz) * rsqrtf(tx * tx + ty * ty + tz * tz), 1e-30f);
     const float d = fmaxf(f - minz, 1e-6f);   // minz: the triangle's least light depth
     const float nb = (float)(1 << depthBits);
     const float q = -log2f(area2 / (d * d)) * (nb / 40.0f) + 0.5f * nb;
@@ -323,6 +329,8 @@ __global__ void __launch_bounds__(256)
         if (depthBits > 0) flush_hist(s_hist, passes * kRadix, orderHist);
         return;
     }
+    const f3 centre = mk3(0.5f * (fr.light.ur[0] + fr.light.dl[0]), 0.5f * (fr.light.ur[1] + fr.light.dl[1]),
+                          0.5f * (fr.light.ur[2] + fr.light.dl[2]));
     const float *M = fr.light.mat;
     const float RFx = fr.light.RF[0], RFy = fr.light.RF[1];
     const float subx = st.subx, suby = st.suby;
@@ -375,7 +383,7 @@ __global__ void __launch_bounds__(256)
             o[1] = make_float4(v1.x, v1.y, v1.z, mxz);
             o[2] = make_float4(v2.x, v2.y, v2.z, 0.0f);
             o[3] = make_float4(mnx, mny, mxx, mxy);
-            order(t, depthBits > 0 ? coverage_bucket(v0, v1, v2, mnz, st.f, depthBits) : 0u);
+            order(t, depthBits > 0 ? coverage_bucket(v0, v1, v2, centre, mnz, st.f, depthBits) : 0u);
             if (mnx <= mxx) store_fast_tri(fast + 4 * (size_t)(fr.triBase + t), fr.light, v0, v1, v2, o[3], mnz, mxz);
         }
         const unsigned b = __ballot_sync(kFullWarp, inLP);

@@ -239,7 +239,8 @@ int fdzb_ctx_set_debug(fdzb_ctx *ctx, int flags);
  * number of pair tests before a sample's light is fully blocked changes.
  *   FDZB_TRI_ORDER_REFERENCE: the reference's order (parity of the sorted lists);
  *   FDZB_TRI_ORDER_COVERAGE (default): largest angular size first (triangle area
- *     over the squared light-depth distance from the far plane to its top vertex). */
+ *     across the line to the light's centre over the squared light-depth distance
+ *     from the far plane to its top vertex). */
 #define FDZB_TRI_ORDER_REFERENCE 0
 #define FDZB_TRI_ORDER_COVERAGE  1
 #define FDZB_TRI_ORDER_DEPTH     FDZB_TRI_ORDER_COVERAGE   /* earlier name of the same value */
