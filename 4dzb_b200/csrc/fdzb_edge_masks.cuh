@@ -574,6 +574,14 @@ template <class R> struct PendingRows {
 };
 template <class R> constexpr int kPending = sizeof(R) == 8 ? 2 : 4;
 
+// Blocks an SM: 8 for the 16-row form without the depth plane, whose 64 registers
+// then spill little (1920 x 1080: 3.02 -> 2.97 ms, 16 mixed frames 25.7 -> 25.0 ms;
+// 9 blocks 3.14); the depth plane's tests need more (6.74 ms at 7, 7.15 at 8).
+// Teams run alone on their SM mostly, so they get the registers (128 x 128 samples,
+// 2000 triangles: 97 us a frame at 5, 107 at 7, 106 at 4).
+template <class R, int DEPTH, int ROWS, int TEAM = 0>
+constexpr int kOccBlocks = TEAM ? 5 : ROWS == 16 && !DEPTH ? 8 : RowWord<R>::kMinBlocks;
+
 // R: the row word (uint32_t for grids up to 32 x 32, u64 up to 64 x 64; a warp
 // per block in the 64-bit form).
 // DEPTH = 1: the pairs also test the triangle's own plane (pair_test).
@@ -590,7 +598,7 @@ template <class R> constexpr int kPending = sizeof(R) == 8 ? 2 : 4;
 // what an early-out of their own would have left out (480 x 270 of the dense
 // frame: 1.7 ms, 6.2 as teams; 2.0 with masks exchanged every 16 triangles).
 template <class R, int DEPTH, int BOX, int COUNT, int ROWS = RowWord<R>::kBits, int TEAM = 0>
-__global__ void __launch_bounds__(RowWord<R>::kWarps * 32, RowWord<R>::kMinBlocks)
+__global__ void __launch_bounds__(RowWord<R>::kWarps * 32, kOccBlocks<R, DEPTH, ROWS, TEAM>)
     k_occlusion(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ states,
                 const int4 *__restrict__ items, int itemCapacity, Counters *ctr,
                 const uint32_t *__restrict__ sortedVals, const int32_t *__restrict__ bss,

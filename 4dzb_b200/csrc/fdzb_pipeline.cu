@@ -1067,7 +1067,7 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     // lane-per-pair schedule only runs square 32-bit grids without the depth
     // plane (the host falls back to lane per sample otherwise)
     typedef RowWord<u64> W64;
-    const int g32 = sm * FDZB_OCC_MINBLOCKS, g64 = sm * W64::kMinBlocks, t64 = W64::kWarps * 32;
+    const int g32 = sm * kOccBlocks<uint32_t, 0, 16>, g64 = sm * W64::kMinBlocks, t64 = W64::kWarps * 32;
 #define FDZB_OCC_LISTS                                                                                       \
     b.frames, b.states, b.items, b.itemCapacity, b.counters, sv, b.binSampleStart, b.binSampleEnd, b.binTriStart, \
         b.binTriEnd, pv, triMask, b.triRec
@@ -1084,7 +1084,7 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
     // team: an item for each block at the most (an item is 32 samples or more of
     // one bin).  The counting forms and those without the cull keep a warp per item.
     const long long mostItems = b.totalSamples / 32 + (b.totalBins < b.totalSamples ? b.totalBins : b.totalSamples);
-    const bool team = b.openBox && !b.countWork && mostItems <= g32;
+    const bool team = b.openBox && !b.countWork && mostItems <= sm * FDZB_OCC_MINBLOCKS;
 #define FDZB_OCC_FORMS(RT, ROWS, G, T)                                                                        \
     do {                                                                                                     \
         if (b.depthPlane && b.openBox) FDZB_OCC(RT, 1, 1, ROWS, G, T);                                        \
