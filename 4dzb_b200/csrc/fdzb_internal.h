@@ -168,6 +168,26 @@ struct DeviceBuffers {
     uint32_t *dbgKeys, *dbgVals, *dbgPKeys, *dbgPVals;
 };
 
+// Which threads of k_reduce's grid (gx x frames x 2 blocks) clear a launch's tables,
+// and by what stride: those of the vertex half's first `blocks` blocks, a few per SM
+// on the host's count.  The whole grid may hold 592 x 65,535 x 2 blocks, more threads
+// than an int numbers.
+struct ClearShare {
+    int first, stride;   // first < 0: the thread clears nothing
+};
+__host__ __device__ inline ClearShare clear_share(int blocks, unsigned bx, unsigned by, unsigned bz, unsigned gx,
+                                                  unsigned threads, unsigned thread)
+{
+    const unsigned block = by * gx + bx;   // below 592 x 65,535
+    if (bz != 1 || block >= (unsigned)blocks) return {-1, 0};
+    return {(int)(block * threads + thread), (int)((unsigned)blocks * threads)};
+}
+// Blocks that clear, of a grid of gx x frames x 2 on `sm` SMs.
+inline int clear_blocks(long long gx, long long frames, int sm)
+{
+    return (int)(gx * frames < 8ll * sm ? gx * frames : 8ll * sm);
+}
+
 // Host side.
 void light_setup(const float rightRadius, const float topRadius, const float position[3],
                  const float viewDir[3], const float upDir[3], int resW, int resH,

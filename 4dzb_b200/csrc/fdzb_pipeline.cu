@@ -48,10 +48,14 @@ struct ClearTargets {
     int32_t *bss, *bse, *bts, *bte;
     int totalBins;
     uint32_t *epochWord, *sortHist;
+    int blocks;   // that clear (clear_share)
 };
 
-__device__ __forceinline__ void clear_launch(const ClearTargets &c, int gid, int stride)
+__device__ __forceinline__ void clear_launch(const ClearTargets &c)
 {
+    const ClearShare share = clear_share(c.blocks, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, blockDim.x, threadIdx.x);
+    const int gid = share.first, stride = share.stride;
+    if (gid < 0) return;
     if (gid == 0) *c.epochWord += 1u;  // launch number: look-back tags of this launch
     for (int i = gid; i < 4 * kSortSlots * kRadix; i += stride) c.sortHist[i] = 0u;
     const uint32_t neg = f2o(-kF32Max), pos = f2o(kF32Max);
@@ -144,8 +148,7 @@ __device__ __forceinline__ void acc_min(uint32_t &a, float v)
 __global__ void __launch_bounds__(kReduceThreads)
     k_reduce(const FrameDesc *__restrict__ frames, FrameState *states, ClearTargets clear)
 {
-    clear_launch(clear, ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
-                 gridDim.x * gridDim.y * gridDim.z * blockDim.x);
+    clear_launch(clear);
     const FrameDesc &fr = frames[blockIdx.y];
     FrameState &st = states[blockIdx.y];
     const float *M = fr.light.mat;
@@ -971,7 +974,7 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
         const int gx = grid_for(maxS > maxV ? maxS : maxV, kReduceThreads, sm * 4);
         k_reduce<<<dim3(gx, nf, 2), kReduceThreads, 0, s>>>(
             b.frames, b.states, {b.binStat, b.binSampleStart, b.binSampleEnd, b.binTriStart, b.binTriEnd, b.totalBins,
-                                 b.epochWord, b.sortHist});
+                                 b.epochWord, b.sortHist, clear_blocks(gx, nf, sm)});
     }
     const bool ordered = b.depthBits > 0 && b.totalTris > 0;
     k_tri_setup<<<dim3(grid_for(maxT, 256, sm * 8), nf), 256, 0, s>>>(
