@@ -226,26 +226,32 @@ void start_states(Engine &e, int nf)
     }
 }
 
+// Both blocks grow together: the old ones stay until the new ones are there, so that
+// after a failed launch the statistics of the one before can still be read.
 int ensure_host(Engine &e, int nf)
 {
-    e.hBases = (int *)((char *)e.hFrames + HostBlock(nf).bases);
-    if (nf <= e.hCap) return FDZB_OK;
-    if (e.pending) cudaStreamSynchronize(e.stream);
-    drop_graph(e);
-    if (e.hFrames) cudaFreeHost(e.hFrames);
-    fdzb::Counters last{};   // of the launch before: its pair count sizes the next one's pair buffers
-    if (e.hCounters) last = *e.hCounters;
-    if (e.hCounters) cudaFreeHost(e.hCounters);
-    e.hFrames = nullptr;
-    e.hCounters = nullptr;
-    e.hCap = 0;
-    const int cap = std::max(nf, 1);
-    FDZB_CUDA(cudaMallocHost(&e.hFrames, HostBlock(cap).bytes));
-    FDZB_CUDA(cudaMallocHost(&e.hCounters, kCountersBytes + sizeof(fdzb::FrameState) * cap));
-    std::memset(e.hCounters, 0, kCountersBytes + sizeof(fdzb::FrameState) * cap);
-    *e.hCounters = last;
-    e.hStates = (fdzb::FrameState *)((char *)e.hCounters + kCountersBytes);
-    e.hCap = cap;
+    if (nf > e.hCap) {
+        const size_t back = kCountersBytes + sizeof(fdzb::FrameState) * (size_t)nf;
+        fdzb::FrameDesc *frames = nullptr;
+        fdzb::Counters *counters = nullptr;
+        cudaError_t err = cudaMallocHost(&frames, HostBlock(nf).bytes);
+        if (err == cudaSuccess) err = cudaMallocHost(&counters, back);
+        if (err != cudaSuccess) {
+            if (frames) cudaFreeHost(frames);
+            cudaGetLastError();
+            return fail(FDZB_ERR_CUDA, std::string("pinned staging: ") + cudaGetErrorString(err));
+        }
+        if (e.pending) cudaStreamSynchronize(e.stream);
+        drop_graph(e);
+        std::memset(counters, 0, back);
+        if (e.hCounters) *counters = *e.hCounters;   // its pair count sizes the next launch's pair buffers
+        if (e.hFrames) cudaFreeHost(e.hFrames);
+        if (e.hCounters) cudaFreeHost(e.hCounters);
+        e.hFrames = frames;
+        e.hCounters = counters;
+        e.hStates = (fdzb::FrameState *)((char *)counters + kCountersBytes);
+        e.hCap = nf;
+    }
     e.hBases = (int *)((char *)e.hFrames + HostBlock(nf).bases);
     return FDZB_OK;
 }
@@ -764,7 +770,8 @@ void launch_stats(const Engine &e, fdzb_frame_stats &o)
     std::memset(&o, 0, sizeof(o));
     o.state = 2;
     long long vs = 0, vt = 0, nb = 0;
-    for (size_t i = 0; i < e.frames.size(); ++i) {
+    // (a list whose launch failed may be longer than the states)
+    for (size_t i = 0; i < std::min(e.frames.size(), (size_t)e.hCap); ++i) {
         const fdzb::FrameState &s = e.hStates[i];
         if (s.state == 2 && s.nValidTris > 0) {
             vs += s.nValidSamples;
@@ -1652,6 +1659,7 @@ int fdzb_batch_get_frame_stats(fdzb_batch *b, int i, fdzb_frame_stats *out)
     if (!out) return fail(FDZB_ERR_INVALID_ARG, "out is NULL");
     if (b->eng.pending) return fail(FDZB_ERR_NOT_READY, "launch not synchronised (fdzb_batch_sync)");
     if (i < 0 || i >= (int)b->eng.frames.size()) return fail(FDZB_ERR_INVALID_ARG, "frame index out of range");
+    if (i >= b->eng.hCap) return fail(FDZB_ERR_NOT_READY, "the launch of this frame list failed");
     frame_stats(b->eng, i, *out);
     return FDZB_OK;
 }
