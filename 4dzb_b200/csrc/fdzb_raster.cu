@@ -19,9 +19,8 @@
 // at slots 2t and 2t+1, with the 16 x 16 pixel tiles their pixel boxes touch (8
 // bytes a slot), and counts the tiles' lists; the lists are laid out (k_rs_lists)
 // and filled (k_rs_scatter); one 256-thread block per tile resolves its pixels
-// and writes each once, cleared or drawn.  Nothing waits on the host: a draw
-// whose lists outgrow their buffer reads the slots' tile boxes instead of the
-// lists (k_rs_tiles), and the next draw finds a larger buffer.
+// and writes each once, cleared or drawn.  The host waits once, for the length of
+// all lists, while they are being laid out (fdzb_raster_draw).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -341,10 +340,13 @@ __global__ void __launch_bounds__(128) k_rs_setup(const float *__restrict__ vtx,
 
 // Lays the tiles' lists out end to end: a block's tiles by a scan of their
 // counts, the blocks in the order in which they arrive (a list's place does not
-// matter; 8,160 tiles: 3 us, 10 us as one block's scan of all tiles).
+// matter; 8,160 tiles: 3 us, 10 us as one block's scan of all tiles).  Hands the
+// draw's counters to the host on the way (pinned memory).
 __global__ void __launch_bounds__(256) k_rs_lists(const int *__restrict__ cnt, const int *__restrict__ more,
-                                                  long long *__restrict__ start, int n, RasterCounters *ctr)
+                                                  long long *__restrict__ start, int n, RasterCounters *ctr,
+                                                  RasterCounters *host)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *host = *ctr;   // k_rs_setup's are final
     __shared__ unsigned long long sWarp[8], sBase;
     const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned long long c = i < n ? (unsigned long long)cnt[i] + (unsigned long long)more[i] : 0ull;
@@ -371,10 +373,8 @@ __global__ void __launch_bounds__(256) k_rs_lists(const int *__restrict__ cnt, c
 
 __global__ void k_rs_scatter(const uint4 *__restrict__ boxes, const uint4 *__restrict__ places, int T, int tilesX,
                              const int *__restrict__ tileCount, const long long *__restrict__ tileStart,
-                             int *__restrict__ tileFill, int *__restrict__ pairs, long long capacity,
-                             const RasterCounters *ctr)
+                             int *__restrict__ tileFill, int *__restrict__ pairs, long long capacity)
 {
-    if ((long long)ctr->pairs > capacity) return;   // the tiles read the boxes instead
     auto put = [&](uint2 b, int slot) {
         const int n = box_tiles(b);
         if (n > 4) {
@@ -438,21 +438,18 @@ struct TileRec {
 // Approximate against exact depth (|z| <= 2): below 2^-19.
 constexpr float kDepthSlack = 1e-5f;
 
-// One block per tile; the tile's list from its buffer or (draws that outgrow
-// it) every slot whose box holds the tile, found by scanning the boxes.  A
-// thread prepares a record, with the warps -- 8 x 4 pixels each -- that have a
-// pixel it can cover (every edge function non-negative at a corner), and each
-// warp goes through its own.  The exact depth (three divisions) is formed
-// only where the approximate one is not clearly behind the pixel's nearest so
-// far.  1920 x 1080, 331k triangles: 705 us as 16 x 2 pixels a warp, every
-// record, 64-bit edge functions; 170 us in this form (70 % of issue slots busy).
+// One block per tile.  A thread prepares a record, with the warps -- 8 x 4
+// pixels each -- that have a pixel it can cover (every edge function non-negative
+// at a corner), and each warp goes through its own.  The exact depth (three
+// divisions) is formed only where the approximate one is not clearly behind the
+// pixel's nearest so far.  1920 x 1080, 331k triangles: 705 us as 16 x 2 pixels a
+// warp, every record, 64-bit edge functions; 170 us in this form (70 % of issue
+// slots busy).
 __global__ void __launch_bounds__(kTile * kTile) k_rs_tiles(const float4 *__restrict__ recs,
-                                                            const uint2 *__restrict__ boxes, int slots,
                                                             const int *__restrict__ tileCount,
                                                             const int *__restrict__ tileMore,
                                                             const long long *__restrict__ tileStart,
-                                                            const int *__restrict__ pairs, long long capacity,
-                                                            const RasterCounters *ctr, int W, int H, int tilesX,
+                                                            const int *__restrict__ pairs, int W, int H, int tilesX,
                                                             int clear, const float *__restrict__ mats, float4 *g0,
                                                             float4 *g1, float4 *g2, float4 *g3, float *depth)
 {
@@ -461,7 +458,6 @@ __global__ void __launch_bounds__(kTile * kTile) k_rs_tiles(const float4 *__rest
     const int tile = blockIdx.x, tx = tile % tilesX, ty = tile / tilesX;
     const int n = tileCount[tile] + tileMore[tile];
     if (n == 0 && !clear) return;
-    const bool listed = (long long)ctr->pairs <= capacity;
     const long long base = tileStart[tile];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wx = 8 * (warp & 1), wy = 4 * (warp >> 1), lx = wx + (lane & 7), ly = wy + (lane >> 3);
@@ -471,26 +467,10 @@ __global__ void __launch_bounds__(kTile * kTile) k_rs_tiles(const float4 *__rest
     const int ox = tx * kTile * 16 + 8, oy = ty * kTile * 16 + 8;   // the tile's first centre
     float bz = __int_as_float(0x7f800000);   // +inf
     int bslot = 0x7fffffff;
-    for (int c0 = 0, scan = 0; c0 < n;) {
+    for (int c0 = 0; c0 < n; c0 += kChunk) {
         __syncthreads();
-        int sl = -1, m;
-        if (listed) {
-            m = min(kChunk, n - c0);
-            if (threadIdx.x < m) sl = pairs[base + c0 + threadIdx.x];
-        } else {
-            if (scan >= slots) break;
-            bool hit = false;
-            if (scan + lane < slots) {
-                const uint2 b = boxes[scan + lane];
-                hit = tx >= (int)(b.x & 0xffffu) && tx <= (int)(b.x >> 16) && ty >= (int)(b.y & 0xffffu) &&
-                      ty <= (int)(b.y >> 16);
-            }
-            const unsigned hits = __ballot_sync(kFullWarp, hit);
-            m = __popc(hits);
-            if (threadIdx.x < m) sl = scan + (int)__fns(hits, 0, threadIdx.x + 1);
-            scan += 32;
-        }
-        c0 += m;
+        const int m = min(kChunk, n - c0);
+        const int sl = threadIdx.x < m ? pairs[base + c0 + threadIdx.x] : -1;
         uint32_t warps = 0;
         if (sl >= 0) {
             const float4 *r = recs + (size_t)kRecF4 * sl;
@@ -629,21 +609,19 @@ static_assert(sizeof(fdzb_raster_stats) == 64, "fdzb_raster_stats layout");
 struct fdzb_raster {
     int device = 0, sms = 148;
     cudaStream_t own = nullptr, stream = nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    float4 *recs = nullptr;
-    uint2 *boxes = nullptr;
-    uint4 *places = nullptr;
-    size_t recSlots = 0, boxSlots = 0, placeSlots = 0;
+    cudaEvent_t e0 = nullptr, e1 = nullptr, counted = nullptr;
+    // records, places and boxes of slotCap slots, one allocation (a cudaMalloc beyond
+    // the small ones takes 0.36 ms, whatever its size)
+    char *slots = nullptr;
+    size_t slotCap = 0;
     // counters, then tileCount, tileMore, tileFill (cleared with them) and tileStart
     char *tiles = nullptr;
     size_t tileCap = 0;
     int *pairs = nullptr;
     size_t pairCap = 0;
-    unsigned long long lastPairs = 0;
     fdzb::RasterCounters *hCtr = nullptr;
     fdzb_raster_stats stats{};
     bool pending = false;
-    bool tooMany = false;   // the last draw had more than 2^31 tile pairs
 };
 
 namespace {
@@ -675,27 +653,16 @@ int grow(void **p, size_t &cap, size_t need, size_t elem)
 constexpr size_t kCtrBytes = 256;
 static_assert(sizeof(fdzb::RasterCounters) <= kCtrBytes, "counters' place before the tile arrays");
 
-// Waits for the draw in flight and takes its counters.
 int finish(fdzb_raster *r)
 {
     if (!r->pending) return FDZB_OK;
     RS_CUDA(cudaEventSynchronize(r->e1));
-    r->pending = false;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, r->e0, r->e1);
-    const fdzb::RasterCounters &c = *r->hCtr;
-    r->lastPairs = c.pairs;
     r->stats.ms = ms;
-    r->stats.sub_triangles = (int64_t)c.subTris;
-    r->stats.dropped = (int64_t)c.dropped;
-    r->stats.tile_pairs = (int64_t)c.pairs;
-    r->stats.bad_indices = (int64_t)c.badIdx;
-    r->stats.bad_materials = (int64_t)c.badMat;
-    r->tooMany = c.pairs > 0x7fffffffull;
+    r->pending = false;
     return FDZB_OK;
 }
-
-int too_many() { return rfail(FDZB_ERR_CAPACITY, "more than 2^31 tile pairs in one draw"); }
 
 }  // namespace
 
@@ -712,6 +679,7 @@ int fdzb_raster_create(fdzb_raster **out, int device)
     r->device = dev;
     if (cudaStreamCreateWithFlags(&r->own, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&r->e0) != cudaSuccess || cudaEventCreate(&r->e1) != cudaSuccess ||
+        cudaEventCreateWithFlags(&r->counted, cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost(&r->hCtr, sizeof(fdzb::RasterCounters)) != cudaSuccess) {
         cudaGetLastError();
         fdzb_raster_destroy(r);
@@ -728,14 +696,13 @@ int fdzb_raster_destroy(fdzb_raster *r)
     if (!r) return FDZB_OK;
     cudaSetDevice(r->device);
     if (r->stream) cudaStreamSynchronize(r->stream);
-    cudaFree(r->recs);
-    cudaFree(r->boxes);
-    cudaFree(r->places);
+    cudaFree(r->slots);
     cudaFree(r->tiles);
     cudaFree(r->pairs);
     if (r->hCtr) cudaFreeHost(r->hCtr);
     if (r->e0) cudaEventDestroy(r->e0);
     if (r->e1) cudaEventDestroy(r->e1);
+    if (r->counted) cudaEventDestroy(r->counted);
     if (r->own) cudaStreamDestroy(r->own);
     delete r;
     return FDZB_OK;
@@ -753,8 +720,7 @@ int fdzb_raster_sync(fdzb_raster *r)
 {
     if (!r) return rfail(FDZB_ERR_INVALID_ARG, "handle is NULL");
     cudaSetDevice(r->device);
-    if (int rc = finish(r)) return rc;
-    return r->tooMany ? too_many() : FDZB_OK;
+    return finish(r);
 }
 
 int fdzb_raster_get_stats(fdzb_raster *r, fdzb_raster_stats *st)
@@ -784,15 +750,21 @@ int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *d)
     if (!d->clear && !d->d_depth) return rfail(FDZB_ERR_INVALID_ARG, "drawing without clear needs the earlier draw's depth buffer");
     cudaSetDevice(r->device);
     if (int rc = finish(r)) return rc;
+    cudaStreamCaptureStatus capture;
+    RS_CUDA(cudaStreamIsCapturing(r->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone)
+        return rfail(FDZB_ERR_CUDA, "a draw waits for its tile-list size and cannot be captured");
 
     const int W = d->W, H = d->H;
     const size_t S = (size_t)W * H;
     const int tilesX = (W + 15) / 16, tilesY = (H + 15) / 16;
     const size_t nTiles = (size_t)tilesX * tilesY;
     const size_t T = (size_t)d->n_tri;
-    if (int rc = grow((void **)&r->recs, r->recSlots, 2 * std::max<size_t>(T, 1), kRecF4 * sizeof(float4))) return rc;
-    if (int rc = grow((void **)&r->boxes, r->boxSlots, 2 * std::max<size_t>(T, 1), sizeof(uint2))) return rc;
-    if (int rc = grow((void **)&r->places, r->placeSlots, 2 * std::max<size_t>(T, 1), sizeof(uint4))) return rc;
+    constexpr size_t kRecBytes = kRecF4 * sizeof(float4), kSlotBytes = kRecBytes + sizeof(uint4) + sizeof(uint2);
+    if (int rc = grow((void **)&r->slots, r->slotCap, 2 * std::max<size_t>(T, 1), kSlotBytes)) return rc;
+    float4 *recs = (float4 *)r->slots;
+    uint4 *places = (uint4 *)(r->slots + kRecBytes * r->slotCap);
+    uint2 *boxes = (uint2 *)(r->slots + (kRecBytes + sizeof(uint4)) * r->slotCap);
     // the four arrays of a capacity of r->tileCap tiles
     if (nTiles > r->tileCap) {
         size_t bytes = 0;
@@ -803,10 +775,6 @@ int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *d)
         if (int rc = grow((void **)&r->tiles, bytes, kCtrBytes + cap * 20 + 8, 1)) return rc;
         r->tileCap = cap;
     }
-    // the tile lists: from the triangles and tiles, or a quarter more than the last draw's
-    const size_t want = std::min<size_t>(std::max<size_t>(6 * T + 4 * nTiles, (size_t)r->lastPairs + (size_t)r->lastPairs / 4), 0x7fffffffull);
-    if (T > 0)
-        if (int rc = grow((void **)&r->pairs, r->pairCap, want, sizeof(int))) return rc;
     RasterCounters *ctr = (RasterCounters *)r->tiles;
     int *tileCount = (int *)(r->tiles + kCtrBytes), *tileMore = tileCount + nTiles, *tileFill = tileMore + nTiles;
     const size_t cleared = kCtrBytes + (12 * nTiles + 7) / 8 * 8;
@@ -823,37 +791,47 @@ int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *d)
         const bool wide = strideF == 8 && d->pos_offset == 0 && d->nrm_offset == 5 && !((uintptr_t)d->d_vtx & 15);
         auto setup = wide ? k_rs_setup<1> : k_rs_setup<0>;
         setup<<<g, 128, 0, s>>>(d->d_vtx, d->n_vtx, strideF, d->pos_offset, d->nrm_offset, d->d_idx, d->n_tri,
-                                d->d_tri_material, d->n_materials, mats, W, H, tilesX, r->recs, r->boxes,
-                                r->places, tileCount, tileMore, ctr);
-        k_rs_lists<<<(unsigned)((nTiles + 255) / 256), 256, 0, s>>>(tileCount, tileMore, tileStart, (int)nTiles, ctr);
-        // A draw whose lists outgrow their buffer scans the slots' boxes, slots / 32
-        // rounds a tile: where that could take long (2^36 slots x tiles: about 0.2
-        // s), the host waits for the lists' size instead and makes the buffer fit.
-        if (2ull * T * nTiles > (1ull << 36)) {
-            RS_CUDA(cudaMemcpyAsync(r->hCtr, ctr, sizeof(RasterCounters), cudaMemcpyDeviceToHost, s));
-            RS_CUDA(cudaStreamSynchronize(s));
-            if (r->hCtr->pairs > 0x7fffffffull) return too_many();
-            if (int rc = grow((void **)&r->pairs, r->pairCap, (size_t)r->hCtr->pairs, sizeof(int))) return rc;
-        }
+                                d->d_tri_material, d->n_materials, mats, W, H, tilesX, recs, boxes, places, tileCount,
+                                tileMore, ctr);
+    }
+    RS_CUDA(cudaGetLastError());
+    // The lists' length sizes their buffer, and a draw of more than 2^31 pairs is
+    // refused before anything is drawn: the host waits for the counters.  A buffer
+    // sized by guess saved nothing (34k triangles: 93 us a draw, 92 with the wait)
+    // and cost draws that outgrew it: 34 ms instead of 2.3 where a view of 100k
+    // triangles moved up to them.
+    *r->hCtr = RasterCounters{};
+    if (T > 0) {
+        k_rs_lists<<<(unsigned)((nTiles + 255) / 256), 256, 0, s>>>(tileCount, tileMore, tileStart, (int)nTiles, ctr, r->hCtr);
+        RS_CUDA(cudaGetLastError());
+        RS_CUDA(cudaEventRecord(r->counted, s));
+        RS_CUDA(cudaEventSynchronize(r->counted));
+    }
+    const RasterCounters c = *r->hCtr;
+    r->stats = fdzb_raster_stats{};
+    r->stats.triangles = d->n_tri;
+    r->stats.sub_triangles = (int64_t)c.subTris;
+    r->stats.dropped = (int64_t)c.dropped;
+    r->stats.tile_pairs = (int64_t)c.pairs;
+    r->stats.bad_indices = (int64_t)c.badIdx;
+    r->stats.bad_materials = (int64_t)c.badMat;
+    r->stats.tiles_x = tilesX;
+    r->stats.tiles_y = tilesY;
+    if (c.pairs > 0x7fffffffull) return rfail(FDZB_ERR_CAPACITY, "more than 2^31 tile pairs in one draw");
+    if (c.pairs > 0) {
+        if (int rc = grow((void **)&r->pairs, r->pairCap, (size_t)c.pairs, sizeof(int))) return rc;
         k_rs_scatter<<<(int)std::min<long long>((d->n_tri + 255) / 256, (long long)sm * 8), 256, 0, s>>>(
-            (const uint4 *)r->boxes, r->places, d->n_tri, tilesX, tileCount, tileStart, tileFill, r->pairs,
-            (long long)r->pairCap, ctr);
-        k_rs_tiles<<<(unsigned)nTiles, 256, 0, s>>>(r->recs, r->boxes, 2 * d->n_tri, tileCount, tileMore, tileStart, r->pairs,
-                                                    (long long)r->pairCap, ctr, W, H, tilesX, d->clear, d->d_materials,
-                                                    (float4 *)d->d_g0, (float4 *)d->d_g1, (float4 *)d->d_g2,
-                                                    (float4 *)d->d_g3, d->d_depth);
+            (const uint4 *)boxes, places, d->n_tri, tilesX, tileCount, tileStart, tileFill, r->pairs, (long long)r->pairCap);
+        k_rs_tiles<<<(unsigned)nTiles, 256, 0, s>>>(recs, tileCount, tileMore, tileStart, r->pairs, W, H, tilesX, d->clear,
+                                                    d->d_materials, (float4 *)d->d_g0, (float4 *)d->d_g1,
+                                                    (float4 *)d->d_g2, (float4 *)d->d_g3, d->d_depth);
     } else if (d->clear) {
         const int g = (int)std::min<size_t>((S + 255) / 256, (size_t)sm * 8);
         k_rs_clear<<<g, 256, 0, s>>>((int)S, (float4 *)d->d_g0, (float4 *)d->d_g1, (float4 *)d->d_g2,
                                      (float4 *)d->d_g3, d->d_depth);
     }
     RS_CUDA(cudaGetLastError());
-    RS_CUDA(cudaMemcpyAsync(r->hCtr, ctr, sizeof(RasterCounters), cudaMemcpyDeviceToHost, s));
     RS_CUDA(cudaEventRecord(r->e1, s));
-    r->stats = fdzb_raster_stats{};
-    r->stats.triangles = d->n_tri;
-    r->stats.tiles_x = tilesX;
-    r->stats.tiles_y = tilesY;
     r->pending = true;
     return FDZB_OK;
 }

@@ -386,11 +386,10 @@ int fdzb_raster_create(fdzb_raster **out, int device);
 int fdzb_raster_destroy(fdzb_raster *r);
 /* stream: a cudaStream_t; NULL = the rasteriser's own stream. */
 int fdzb_raster_set_stream(fdzb_raster *r, void *stream);
-/* Enqueues one draw (after waiting for the handle's previous one) and returns
- * with the rasterisation in flight; fdzb_raster_sync waits for it.  Draws of
- * very many triangles on very large views wait once on the stream for the
- * tile-list size.  More than 2^31 (sub-triangle, tile) pairs in one draw:
- * FDZB_ERR_CAPACITY, from the draw or from the sync. */
+/* Enqueues one draw (after waiting for the handle's previous one).  Waits once on
+ * the stream for the tile-list size, then returns with the rasterisation in
+ * flight; fdzb_raster_sync waits for it.  More than 2^31 (sub-triangle, tile)
+ * pairs in one draw: FDZB_ERR_CAPACITY, and nothing is drawn. */
 int fdzb_raster_draw(fdzb_raster *r, const fdzb_raster_desc *desc);
 int fdzb_raster_sync(fdzb_raster *r);
 int fdzb_raster_get_stats(fdzb_raster *r, fdzb_raster_stats *stats);
