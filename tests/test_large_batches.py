@@ -104,6 +104,7 @@ def test_thousands_of_frames_equal_one(cuda_ok, fdzb, scenes, frames, vertices):
     for _ in range(2):
         shadow.fill_(-1.0)
         masks.fill_(-1)
+        torch.cuda.synchronize()   # the batch has a stream of its own
         b.launch(desc)
         assert torch.equal(shadow.view(torch.int32), want[0].view(torch.int32).reshape(1, -1).expand(frames, -1))
         assert torch.equal(masks, want[1].reshape(1, -1).expand(frames, -1))
