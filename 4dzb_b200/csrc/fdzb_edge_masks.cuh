@@ -577,10 +577,18 @@ template <class R> constexpr int kPending = sizeof(R) == 8 ? 2 : 4;
 // Blocks an SM: 8 for the 16-row form without the depth plane, whose 64 registers
 // then spill little (1920 x 1080: 3.02 -> 2.97 ms, 16 mixed frames 25.7 -> 25.0 ms;
 // 9 blocks 3.14); the depth plane's tests need more (6.74 ms at 7, 7.15 at 8).
-// Teams run alone on their SM mostly, so they get the registers (128 x 128 samples,
-// 2000 triangles: 97 us a frame at 5, 107 at 7, 106 at 4).
+// Teams get more registers (128 x 128 samples, 2000 triangles: 97 us a frame at 5,
+// 107 at 7, 106 at 4).
 template <class R, int DEPTH, int ROWS, int TEAM = 0>
 constexpr int kOccBlocks = TEAM ? 5 : ROWS == 16 && !DEPTH ? 8 : RowWord<R>::kMinBlocks;
+
+// Items an SM, at the most, of a launch that runs as teams; not the resident blocks,
+// which take the items beyond them as they finish.  As teams / a warp an item, us a
+// frame: 5.2 items an SM, 2000 triangles 105 / 142, 8000 167 / 347; 7.0 items, 400
+// triangles 95 / 102, 8000 195 / 326.  Above the line teams still win at 9.1 items (8000
+// triangles 208 / 398) and at 13.8 (2000: 121 / 140), and lose by far at 55 (the 480 x
+// 270 view); where between is not measured.
+constexpr int kTeamItems = 7;
 
 // R: the row word (uint32_t for grids up to 32 x 32, u64 up to 64 x 64; a warp
 // per block in the 64-bit form).
@@ -592,11 +600,11 @@ constexpr int kOccBlocks = TEAM ? 5 : ROWS == 16 && !DEPTH ? 8 : RowWord<R>::kMi
 // ROWS: light rows a lane's mask holds in shared memory (RowWord<R>::kBits, or
 // 16 for launches whose grids have at most 16 rows of at most 31 columns).
 // TEAM = 1: a block's warps take one item together, a chunk of its triangles
-// each in turn, and OR their masks.  For launches with no more items than the
-// chip holds blocks, which last as long as their longest item: 128 x 96 samples,
-// 400 triangles: 104 -> 94 us a frame.  Not beyond: with more items the warps do
-// what an early-out of their own would have left out (480 x 270 of the dense
-// frame: 1.7 ms, 6.2 as teams; 2.0 with masks exchanged every 16 triangles).
+// each in turn, and OR their masks.  For launches of few items (kTeamItems), which
+// last as long as their longest item: 128 x 96 samples, 400 triangles: 104 -> 94 us a
+// frame.  With many items the warps do what an early-out of their own would have
+// left out (480 x 270 of the dense frame: 1.7 ms, 6.2 as teams; 2.0 with masks
+// exchanged every 16 triangles).
 template <class R, int DEPTH, int BOX, int COUNT, int ROWS = RowWord<R>::kBits, int TEAM = 0>
 __global__ void __launch_bounds__(RowWord<R>::kWarps * 32, kOccBlocks<R, DEPTH, ROWS, TEAM>)
     k_occlusion(const FrameDesc *__restrict__ frames, const FrameState *__restrict__ states,

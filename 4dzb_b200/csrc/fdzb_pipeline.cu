@@ -1087,10 +1087,10 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
         else                                                                                                 \
             k_occlusion<RT, DP, BX, 0, ROWS><<<G, T, 0, s>>>(FDZB_OCC_LISTS, b.triFast, b.totalTris, b.totalBins, nf); \
     } while (0)
-    // team: an item for each block at the most (an item is 32 samples or more of
-    // one bin).  The counting forms and those without the cull keep a warp per item.
+    // team: few items (kTeamItems; an item is 32 samples or more of one bin, or a
+    // bin's last).  The counting forms and those without the cull keep a warp per item.
     const long long mostItems = b.totalSamples / 32 + (b.totalBins < b.totalSamples ? b.totalBins : b.totalSamples);
-    const bool team = b.openBox && !b.countWork && mostItems <= sm * FDZB_OCC_MINBLOCKS;
+    const bool team = b.openBox && !b.countWork && mostItems <= sm * kTeamItems;
 #define FDZB_OCC_FORMS(RT, ROWS, G, T)                                                                        \
     do {                                                                                                     \
         if (b.depthPlane && b.openBox) FDZB_OCC(RT, 1, 1, ROWS, G, T);                                        \
