@@ -168,8 +168,14 @@ int ensure_arena(Engine &e, int nf, long long S, long long T, long long NB, long
             e.arena = nullptr;
             e.arenaBytes = 0;
         }
-        const size_t bytes = align_up(need + need / 8, 1 << 20);
+        // room to grow into, or what the launch needs where that is all there is
+        size_t bytes = align_up(need + need / 8, 1 << 20);
         cudaError_t err = cudaMalloc(&e.arena, bytes);
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            bytes = align_up(need, 1 << 20);
+            err = cudaMalloc(&e.arena, bytes);
+        }
         if (err != cudaSuccess) {
             e.arena = nullptr;
             cudaGetLastError();

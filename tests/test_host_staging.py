@@ -1,10 +1,11 @@
-"""A launch whose pinned staging cannot grow, on the CPU.
+"""Launches whose pinned staging or device arena cannot grow, on the CPU.
 
 fdzb_api.cpp is built against a small stand-in for the CUDA runtime: device and
 pinned memory are host memory, copies happen at once, the kernels do nothing, and
 a pinned allocation can be made to fail.  A batch that needs more staging than
 there is fails with an error; what the handle knew of the launch before can still
-be read afterwards, frames beyond it are refused, and the next launch works.
+be read afterwards, frames beyond it are refused, and the next launch works.  An arena is
+allocated with an eighth to spare, and without where that does not fit.
 """
 import json
 import os
@@ -21,10 +22,16 @@ FAKE = r"""
 #include "fdzb_internal.h"
 
 extern "C" int fake_pinned_left = 1 << 30;   // pinned allocations until one fails
+extern "C" size_t fake_device_limit = ~(size_t)0, fake_device_asked = 0;   // bytes of one allocation
 static int s_object;
 
 extern "C" {
-cudaError_t cudaMalloc(void **p, size_t n) { return (*p = std::calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaMalloc(void **p, size_t n)
+{
+    if (n > fake_device_limit) { *p = nullptr; return cudaErrorMemoryAllocation; }
+    fake_device_asked = n;
+    return (*p = std::calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation;
+}
 cudaError_t cudaFree(void *p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned)   // cudaMallocHost of typed pointers
 {
@@ -84,7 +91,7 @@ cudaError_t check_division(unsigned long long, unsigned long long, unsigned long
 }
 """
 
-DRIVE = r"""
+SETUP = r"""
 import ctypes, importlib, json, sys
 sys.path.insert(0, sys.argv[1])
 m = importlib.import_module("4dzb_b200")
@@ -100,14 +107,17 @@ lib.fdzb_batch_destroy.argtypes = [vp]
 mem = (ctypes.c_float * 4096)()
 at = (ctypes.addressof(mem) + 63) // 64 * 64
 
-def frames(n):
+def frames(n, tris=1):
     light = importlib.import_module("4dzb_b200.scenes").Light(right_radius=1.0, top_radius=1.0, n=4)
-    return (m.FrameDesc * n)(*[m.frame_desc(at, at, 4, 4, at, 3, at, 1, light, at, None, bins=4) for _ in range(n)])
+    return (m.FrameDesc * n)(*[m.frame_desc(at, at, 4, 4, at, 3, at, tris, light, at, None, bins=4) for _ in range(n)])
 
-b = vp()
-assert lib.fdzb_batch_create(ctypes.byref(b), 0) == 0
-assert lib.fdzb_batch_set_graph(b, 0) == 0
-ms, out = ctypes.c_float(), []
+def batch():
+    b = vp()
+    assert lib.fdzb_batch_create(ctypes.byref(b), 0) == 0
+    assert lib.fdzb_batch_set_graph(b, 0) == 0
+    return b
+
+b, ms, out = batch(), ctypes.c_float(), []
 
 def totals():
     s = m.BatchStats()
@@ -118,9 +128,11 @@ def frame(i):
     rc = lib.fdzb_batch_get_frame_stats(b, i, ctypes.byref(s))
     return [rc, s.valid_samples if rc == 0 else 0]
 
-def launch(n):
-    return lib.fdzb_batch_launch(b, frames(n), n, ctypes.byref(ms))
+def launch(n, tris=1):
+    return lib.fdzb_batch_launch(b, frames(n, tris), n, ctypes.byref(ms))
+"""
 
+STAGING = r"""
 out.append([launch(2), totals(), frame(0), frame(1)])
 for fails in (0, 1):             # the first block of the larger launch, then its second
     left.value = fails
@@ -129,6 +141,16 @@ for fails in (0, 1):             # the first block of the larger launch, then it
 out.append([launch(2), totals(), frame(1)])
 out.append([launch(3000), totals(), frame(2999)])
 assert lib.fdzb_batch_destroy(b) == 0
+print(json.dumps(out))
+"""
+
+ARENA = r"""
+limit, asked = (ctypes.c_size_t.in_dll(lib, k) for k in ("fake_device_limit", "fake_device_asked"))
+assert launch(1, 20000) == 0
+spare = asked.value                       # the need and an eighth, whole megabytes
+for limit.value in (spare - 1, spare * 8 // 9 - (2 << 20)):
+    b = batch()
+    out.append([launch(1, 20000), asked.value < spare])
 print(json.dumps(out))
 """
 
@@ -148,15 +170,26 @@ def library(tmp_path_factory):
     return out
 
 
-def test_statistics_outlive_a_launch_without_staging(library, tmp_path):
+def _drive(library, tmp_path, steps):
     script = tmp_path / "drive.py"
-    script.write_text(DRIVE)
+    script.write_text(SETUP + steps)
     r = subprocess.run([sys.executable, str(script), ROOT, library], capture_output=True, text=True,
                        env=dict(os.environ, MALLOC_PERTURB_="165"))
     assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
-    first, no_frames, no_states, again, large = json.loads(r.stdout)
+    return json.loads(r.stdout)
+
+
+def test_statistics_outlive_a_launch_without_staging(library, tmp_path):
+    first, no_frames, no_states, again, large = _drive(library, tmp_path, STAGING)
     assert first == [0, [0, 14], [0, 100], [0, 101]]
     for failed in (no_frames, no_states):
         assert failed == [True, [0, 14], [0, 100], [0, 101], True]
     assert again == [0, [0, 14], [0, 101]]
     assert large == [0, [0, 21000], [0, 3099]]
+
+
+def test_an_arena_without_room_to_spare(library, tmp_path):
+    """The launch runs where its need fits and the spare eighth does not; below the need it is refused."""
+    fits, refused = _drive(library, tmp_path, ARENA)
+    assert fits == [0, True]
+    assert refused[0] == -4   # FDZB_ERR_NO_MEMORY
