@@ -640,11 +640,16 @@ int grow(void **p, size_t &cap, size_t need, size_t elem)
     if (*p) cudaFree(*p);
     *p = nullptr;
     cap = 0;
+    // a quarter to spare, or what the draw needs where that is all there is
     size_t n = need + need / 4 + 64;
     if (cudaMalloc(p, n * elem) != cudaSuccess) {
-        *p = nullptr;
         cudaGetLastError();
-        return rfail(FDZB_ERR_NO_MEMORY, "device allocation failed");
+        n = need;
+        if (cudaMalloc(p, n * elem) != cudaSuccess) {
+            *p = nullptr;
+            cudaGetLastError();
+            return rfail(FDZB_ERR_NO_MEMORY, "device allocation failed");
+        }
     }
     cap = n;
     return FDZB_OK;
