@@ -57,12 +57,14 @@
 // of dir) could differ (gs).
 //
 // Measured (B200, CUDA events, occlusion stage), against the reference's test
-// for every pair with its quotients from hoisted reciprocals (the same masks):
-// 1920 x 1080 with 200k triangles, 16 x 16 light 5.33 -> 4.17 ms, with 20k
-// triangles 6.00 -> 3.61 ms, 64 x 48 light 26.5 -> 19.7 ms; 1280 x 720, 50k
-// triangles up to and behind the light with the depth plane 25.3 -> 7.3 ms;
-// 3840 x 2160, 2M triangles, 32 x 32 light (whole frame) 1334 -> 382 ms.
-// Issue-bound: 82 % of issue slots busy, the ALU pipe 64 %, 17.7 of 32 lanes.
+// for every pair with its quotients from hoisted reciprocals (the same masks), and
+// after the steps noted below and the coverage order (k_tri_setup):
+// 1920 x 1080 with 200k triangles, 16 x 16 light 5.33 -> 4.17 -> 2.95 ms, with 20k
+// triangles 6.00 -> 3.61 -> 3.28 ms, 64 x 48 light 26.5 -> 19.7 -> 14.3 ms; 1280 x
+// 720, 50k triangles up to and behind the light with the depth plane 25.3 -> 7.3 ->
+// 6.70 ms; 3840 x 2160, 2M triangles, 32 x 32 light (whole frame) 1334 -> 382 -> 344 ms.
+// Issue-bound (the first of these frames): 84 % of issue slots busy, the ALU pipe
+// 66 %, 19.1 of 32 lanes.
 #pragma once
 #include "fdzb_occlusion.cuh"
 
@@ -363,7 +365,8 @@ __device__ __forceinline__ R fast_pair(const FastTri &T, const FastSample &s, co
             if (!(d12 > 0.0f && err < 0.25f)) return open;
         }
     }
-    const float volume = dz0 * dz1 * dz2 * (w * gs);   // >= |dir| h^2 / Vol
+    // at most |dir| h^2 / Vol: beyond espK, |dir| is not below esp and nothing is skipped
+    const float volume = dz0 * dz1 * dz2 * (w * gs);
     if (!(volume > s.espK)) {
         const int tri = (int)(*triAt & triMask);
         if ((unsigned)tri >= (unsigned)totalTris || self_skip(rec, tri, pos, esp)) return 0;
@@ -382,7 +385,7 @@ __device__ __forceinline__ R fast_pair(const FastTri &T, const FastSample &s, co
     R *row = &rows[rFirst][lane];
     R bit = R(1) << rFirst;
     // A row's cost is its issue slots, those of the integer and compare pipe most
-    // (64 % of its rate at 82 % of the issue rate): the row number counts the loop, and
+    // (66 % of its rate at 84 % of the issue rate): the row number counts the loop, and
     // both ends are rounded as a pair.  1920 x 1080, 16 x 16 light: 4.15 -> 3.93 ms
     // (with a counter of its own 4.06; the lines as pairs too: 4.27).
     float rf = (float)rFirst;

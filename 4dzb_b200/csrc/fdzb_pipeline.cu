@@ -1031,8 +1031,9 @@ cudaError_t run_pipeline(const DeviceBuffers &b, int maxS, int maxT, int maxV, c
         // of few triangles still spreads over the SMs (2k triangles: pairs
         // 0.159 -> 0.074 ms against tiles of 256; HD: 0.305 -> 0.277 ms);
         // above, tiles of 256 (64 frames, 8.9M triangles: 7.1 ms against 8.4
-        // ms with tiles of 64).  Up to 8 blocks per SM: the sweeps wait on
-        // bin-statistics loads, so more resident warps hide more of that latency.
+        // ms with tiles of 64).  The sweeps wait on bin-statistics loads, which
+        // resident warps hide: 4 blocks an SM at a time (64 registers a thread, all
+        // of its threads' worth of them), up to 8 in the grid.
         // Up to kTriTiny triangles an SM: tiles of 8, a triangle a warp (pairs stage,
         // 400 triangles 0.030 -> 0.023 ms, 1024: 0.032 -> 0.026; 7001 the same either
         // way, 50k in tiles of 8: 0.24 -> 0.34 ms).

@@ -25,10 +25,11 @@ __device__ __forceinline__ float3 f3n(float3 v)
     return make_float3(v.x * r, v.y * r, v.z * r);
 }
 
-// ONE: a single light sample, as the application shades with: HBM-bound, so 8
-// blocks an SM with all five of a pixel's loads in flight (1920 x 1080: 39 -> 26
-// us, 6.6 TB/s; 6 blocks 34 us).  More samples: ALU-bound (the powers), where the
-// 40 registers of 6 blocks are the faster form (64 samples: 559 us, 639 at 8).
+// ONE: a single light sample, as the application shades with: HBM-bound, so all
+// five of a pixel's loads are in flight at once (1920 x 1080, 174 MB: a call on inputs
+// that the L2 does not hold 40.1 -> 32.4 us, 5.4 TB/s; on the same ones again 39 -> 26;
+// 6 blocks an SM instead of 8: 31.4 and 25).  More samples: ALU-bound (the powers),
+// where the 40 registers of 6 blocks are the faster form (64 samples: 559 us, 639 at 8).
 template <int ONE>
 __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_shade(int npix, const float4 *__restrict__ g0,
                                                const float4 *__restrict__ g1, const float4 *__restrict__ g2,

@@ -287,8 +287,9 @@ int fdzb_measure_alu_rate(double *lane_ops_per_second);
 
 /* Device self-check of a row quotient -D / B from a hoisted reciprocal RN(1/B)
  * by two Markstein correction steps, the reciprocal itself from the hardware
- * approximation and one
- * Newton-Raphson step.  Compares that reciprocal with __frcp_rn for every
+ * approximation and one Newton-Raphson step.  No kernel takes that quotient any more
+ * (rows that need the reference's quotient divide), so nothing depends on the
+ * result; it remains a check of the device's FP32 arithmetic.  Compares that reciprocal with __frcp_rn for every
  * float of the admitted range (|B| in [2^-100, 2^40), 2.35e9 values), then
  * runs `trials` trials of three cases each (random operands over the admitted
  * ranges, quotients next to rounding midpoints, quotients at small integers)
