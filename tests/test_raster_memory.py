@@ -74,8 +74,9 @@ def library(tmp_path_factory):
     out = str(tmp / "libraster.so")
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     env = {k: v for k, v in os.environ.items() if k not in ("CC", "CXX")}
+    # -Bsymbolic: the stand-in, whatever runtime this process has loaded
     r = subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O1", "-std=c++17", "-Xcompiler", "-fPIC",
-                        "-shared", "-cudart", "none", "-I", os.path.join(ROOT, "include"),
+                        "-shared", "-cudart", "none", "-Xlinker", "-Bsymbolic", "-I", os.path.join(ROOT, "include"),
                         os.path.join(ROOT, "4dzb_b200", "csrc", "fdzb_raster.cu"), str(tmp / "fake.cpp"), "-o", out],
                        capture_output=True, text=True, env=env)
     assert r.returncode == 0, r.stderr
